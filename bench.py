@@ -15,11 +15,14 @@ run.  Working set 1.2 GB >> 126 MB L2, so no L2 flush is needed between steps.
   e2e    the same metric through the public API with host buffers: operator
          upload (H2D), K batches with their sampled waveforms (H2D) and energy
          samples / probe traces (D2H), and the final read_fields (D2H).
-  roofline  the H and E update kernels (each ~half the step): 60 algorithmic
-         bytes per cell per launch (120 B per cell-step; --compressed 37,
-         --storage f16/bf16 42, both 19: see kernel_bytes), timed with CUDA
-         events around every launch on the engine's stream in a profiling
-         batch of the same workload run after the timed region.
+  roofline  the fused two-step passes (the default): every field read and
+         written and a material id read once per two steps, 49 bytes per cell
+         and pass (--storage f16/bf16 25); the kernel works out of the
+         register file and shared memory, so its fraction of the HBM peak is
+         low where the separate H and E kernels' (--kernels register and the
+         like; 60 bytes per cell and launch, see kernel_bytes) is high.  Timed
+         with CUDA events around every launch on the engine's stream in a
+         profiling batch of the same workload run after the timed region.
   cpu_baseline  the oracle's C++ restatements of the reference's CPU engines
          (the Rayon engine's cell loop and the SIMD engine's z-lines, OpenMP
          over x-planes, -O3 / AVX2, same arithmetic and bits): the faster of
@@ -58,6 +61,14 @@ def kernel_bytes(storage: str, compressed: bool) -> float:
     material id, the table being in shared memory)."""
     elem = 4 if storage == "f32" else 2
     return 9 * elem + (1 if compressed else 24)
+
+
+def pass_bytes(storage: str) -> float:
+    """Algorithmic bytes per cell of one fused pass (two steps): the six
+    fields read and written once and a one-byte material id."""
+    return 12 * (4 if storage == "f32" else 2) + 1
+
+
 STEPS_PER_BENCH_STEP = 1000
 METRIC = "MCells/s (Yee FDTD throughput, % of HBM roofline)"
 
@@ -198,7 +209,7 @@ def run_device(oe, wl, args, torch, dist):
     info = eng.launch_info()
     tune = {}
     for r in eng.tune_report():  # fastest timed shape of each kernel family
-        k = ("register", "staged", "staged_split", "register_zsplit", "register_pipe")[r["kind"]]
+        k = ("register", "staged", "staged_split", "register_zsplit", "register_pipe", "fused")[r["kind"]]
         per = r["ms"] / max(r["reps"], 1)
         if k not in tune or per < tune[k]["ms_per_step"]:
             tune[k] = {"ms_per_step": per, "threads": r["threads"], "ichunk": r["ichunk"], "extra": r["extra"]}
@@ -449,6 +460,10 @@ def main():
     kernel_avg = max(d["h_avg_s"], d["e_avg_s"])
     dominant = "k_update_h" if d["h_avg_s"] >= d["e_avg_s"] else "k_update_e"
     per_kernel = kernel_bytes(args.storage, args.compressed)
+    per_step = 2 * per_kernel
+    if d["launch"]["staged"] == 5:
+        dominant, per_kernel = "k_fused", pass_bytes(args.storage)
+        per_step = per_kernel / 2
     achieved = per_kernel * wl.cells / kernel_avg / 1e9
     traffic = None
     prof_path = os.path.join(ROOT, "profiles", "traffic.json")
@@ -464,13 +479,13 @@ def main():
     # the sweep half of the metric: one GPU (at N > 1 the ranks would run
     # replicas of the same sweep, which adds nothing)
     sweep = None if (args.no_sweep or world > 1) else sweep_metric()
-    step_gbs = 2 * per_kernel * wl.cells * steps_total / t_dev / 1e9 / world
+    step_gbs = per_step * wl.cells * steps_total / t_dev / 1e9 / world
     line = {
         "metric": METRIC, "value": value, "unit": "MCells/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": t_dev / args.steps * 1e3, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": config,
-        "hbm_fraction_step": step_gbs / hbm,
+        "hbm_fraction_step": step_gbs / hbm, "bytes_per_cell_step": per_step,
         "roofline": {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": hbm,
                      "peak_source": peak_src, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": traffic,

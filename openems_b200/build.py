@@ -16,7 +16,8 @@ ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "liboems_b200.so")
 SOURCES = ["csrc/engine.cu", "csrc/host.cpp", "csrc/noalloc.cu", "csrc/sweep.cpp", "csrc/predictor_kernels.cu",
            "csrc/cylindrical.cu"]
-HEADERS = ["csrc/yee_kernels.cuh", "csrc/yee_pipe.cuh", "csrc/yee_tma.cuh", "csrc/mur.cuh", "csrc/lumped_ade.cuh",
+HEADERS = ["csrc/yee_kernels.cuh", "csrc/yee_pipe.cuh", "csrc/yee_tma.cuh", "csrc/yee_fused.cuh",
+           "csrc/fused_host.cuh", "csrc/mur.cuh", "csrc/lumped_ade.cuh",
            "csrc/fd_nf2ff.cuh", "csrc/upml.cuh", "csrc/interface.cuh", "csrc/gemm_tc.cuh", "../include/oems.h",
            "../include/oems_host.h", "../include/oems_predictor.h"]
 
@@ -25,7 +26,7 @@ NVCC_FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-O2,-fvisibility=hidden",
     "--expt-relaxed-constexpr",
-    "-shared",
+    "-shared", "--split-compile=0",
 ]
 
 

@@ -40,6 +40,7 @@
 #include "fd_nf2ff.cuh"
 #include "upml.cuh"
 #include "interface.cuh"
+#include "yee_fused.cuh"
 
 namespace oems {
 
@@ -558,6 +559,44 @@ struct UpmlHost {
   DevBuf<float> coef, flux;          // [E coef | H coef], [E flux | H flux]
 };
 
+// Fused passes (yee_fused.cuh, fused_host.cuh).
+using FusedKernel = void (*)(FusedArgs);
+struct FusedPlan {
+  int steps = 1, nbox = 0, ncpml = 0;  // boxes; the first ncpml meet slabs
+  FusedBox box[kFusedMaxBox];
+  // [0] the launch of the boxes clear of the slabs, [1] of the others
+  int nt[2] = {0, 0}, items[2] = {0, 0}, pairs = 0;
+  size_t smem[2] = {0, 0};
+  double cost = 0.0;
+};
+struct FusedKey {
+  int dev, nx, ny, nz, id_bytes, ntable, prof, mode;
+  bool operator<(const FusedKey& o) const {
+    return std::tie(dev, nx, ny, nz, id_bytes, ntable, prof, mode) <
+           std::tie(o.dev, o.nx, o.ny, o.nz, o.id_bytes, o.ntable, o.prof, o.mode);
+  }
+};
+struct FusedHost {
+  int state = 0;      // 0 not looked at, 1 prepared, -1 not for this engine
+  bool use = false;   // this batch runs as fused passes
+  bool tuned = false;
+  int parity = 0;     // which of the two buffer sets is current
+  DevBuf<char> alt;   // the buffers the next pass writes
+  DevBuf<float> psi;
+  const void* ids = nullptr;
+  const float* table = nullptr;
+  int id_bytes = 0, ntable = 0;
+  DevBuf<uint8_t> own_ids;
+  DevBuf<float> own_table;
+  FusedPlan plan[2];
+  DevBuf<int> src_i;         // plane offsets, keys, element / direction / kind
+  DevBuf<long long> src_q;   // first sample and sample count
+  int src_lo = 0, src_hi = 0;
+  DevBuf<int> tap_i;
+  int ntap = 0, tap_lo = 0, tap_hi = 0;
+  DevBuf<float> taps;
+};
+
 }  // namespace oems
 
 struct oems_engine {
@@ -625,8 +664,10 @@ struct oems_engine {
   oems::Geom gs{};  // shell segments of a split shape
   bool tuned = false;
   std::vector<oems_tune_entry> tune_report;  // candidates timed by the last tuning
+  oems::FusedHost fus;
 
-  // graphs keyed by span length; invalidated when any baked pointer changes
+  // graphs keyed by span length and current buffers; invalidated when any
+  // baked pointer changes
   std::map<int, cudaGraphExec_t> graphs;
   uint64_t graph_epoch = 0, built_epoch = ~0ull;
 
@@ -1015,16 +1056,20 @@ static oems_status size_grid(oems_engine* en, LaunchShape& s) {
   return OEMS_OK;
 }
 
-static void apply_shape(oems_engine* en, const LaunchShape& s) {
-  if (s.fork && !en->side) {
-    // created on first use; failures leave the shape unforked
+// The second stream and its events, created on first use; false: not to be had.
+static bool side_stream(oems_engine* en) {
+  if (!en->side) {
     if (cudaStreamCreateWithFlags(&en->side, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&en->fork_ev, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&en->join_ev, cudaEventDisableTiming) != cudaSuccess)
       cudaGetLastError();
   }
+  return en->side && en->fork_ev && en->join_ev;
+}
+
+static void apply_shape(oems_engine* en, const LaunchShape& s) {
   en->shape = s;
-  if (s.fork && !(en->side && en->fork_ev && en->join_ev)) en->shape.fork = false;
+  if (s.fork && !side_stream(en)) en->shape.fork = false;
   en->g = s.zsplit ? make_interior_geom(en, s.block, s.ichunk) : make_geom(en, s.block, s.ichunk);
   en->g.pf = (s.tma || s.pipe) ? 0 : s.pf;
   if (s.split || s.zsplit) en->gs = make_shell_geom(en, s.sh_block, s.sh_ichunk, s.zsplit);
@@ -1140,6 +1185,7 @@ static bool need_post(const oems_engine* en) { return post_kernels(en) > 0; }
 static cudaError_t launch_fd(oems_engine* en, int local) {
   for (FieldDftHost& d : en->fdumps) {
     FieldDftArgs a = d.args;
+    for (size_t k = 0; k < d.comps.size(); ++k) a.f[k] = en->at((size_t)d.comps[k]);
     a.tw = d.tab->tw.p;
     a.sampled = d.tab->sampled.p;
     a.d_base = en->d_base.p;
@@ -1148,6 +1194,10 @@ static cudaError_t launch_fd(oems_engine* en, int local) {
   }
   for (Nf2ffHost& b : en->boxes) {
     Nf2ffAccArgs a = b.args;
+    for (int c = 0; c < 3; ++c) {
+      a.e[c] = en->E(c);
+      a.h[c] = en->H(c);
+    }
     a.tw = b.tab->tw.p;
     a.sampled = b.tab->sampled.p;
     a.d_base = en->d_base.p;
@@ -1203,7 +1253,18 @@ static int second_order_disp(const oems_engine* en) {
   return k;
 }
 
+// Extension arguments on the current field buffers (a fused pass swaps them).
+static void current_fields(oems_engine* en) {
+  for (int c = 0; c < 3; ++c) {
+    en->mur.args.e[c] = en->E(c);
+    for (DispHost& d : en->disp) d.args.e[c] = en->E(c);
+    en->upml.e.f[c] = en->E(c);
+    en->upml.h.f[c] = en->H(c);
+  }
+}
+
 static cudaError_t launch_pre_e(oems_engine* en) {
+  current_fields(en);
   if (en->mur.on) {
     k_mur_pre<<<blocks_for(en->mur.args.total, 256), 256, 0, en->stream>>>(en->mur.args);
     cudaError_t e = cudaGetLastError();
@@ -1217,6 +1278,7 @@ static cudaError_t launch_pre_e(oems_engine* en) {
 }
 
 static cudaError_t launch_post_e(oems_engine* en) {
+  current_fields(en);
   if (en->upml.on) {
     cudaError_t e = launch_upml(en, false, false);
     if (e != cudaSuccess) return e;
@@ -1255,6 +1317,7 @@ static int kernels_per_step(const oems_engine* en) {
 
 // Launches `steps` timesteps directly (no graph).
 static cudaError_t launch_upml(oems_engine* en, bool h, bool pre) {
+  current_fields(en);
   const UpmlArgs& a = h ? en->upml.h : en->upml.e;
   const int b = blocks_for(a.total, 256);
   if (pre)
@@ -1416,20 +1479,31 @@ static oems_status launch_steps_profiled(oems_engine* en, int steps) {
   return OEMS_OK;
 }
 
+static std::mutex& tune_mutex();
+static oems_status launch_steps_fused(oems_engine* en, int steps);
+static uint64_t fused_launches(const oems_engine* en, int steps);
+static void fused_swap(oems_engine* en);
+static int fused_max_steps(const oems_engine* en);
+
 static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
   if (en->built_epoch != en->graph_epoch) {
     drop_graphs(en);
     en->built_epoch = en->graph_epoch;
   }
-  auto it = en->graphs.find(steps);
+  const int key = 2 * steps + en->fus.parity;
+  auto it = en->graphs.find(key);
   if (it != en->graphs.end()) {
     *out = it->second;
+    if (en->fus.use) {
+      const int most = fused_max_steps(en);
+      if ((steps + most - 1) / most & 1) fused_swap(en);
+    }
     return OEMS_OK;
   }
   if (en->graphs.size() >= 8) drop_graphs(en);
   cudaGraph_t graph = nullptr;
   OEMS_CUDA(cudaStreamBeginCapture(en->stream, cudaStreamCaptureModeThreadLocal));
-  oems_status st = launch_steps_direct(en, steps);
+  oems_status st = en->fus.use ? launch_steps_fused(en, steps) : launch_steps_direct(en, steps);
   cudaError_t ce = cudaStreamEndCapture(en->stream, &graph);
   if (st != OEMS_OK) {
     if (graph) cudaGraphDestroy(graph);
@@ -1440,7 +1514,7 @@ static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
   ce = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   if (ce != cudaSuccess) return fail(OEMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-  en->graphs[steps] = exec;
+  en->graphs[key] = exec;
   *out = exec;
   return OEMS_OK;
 }
@@ -1452,7 +1526,13 @@ static oems_status run_span(oems_engine* en, long long base, int steps) {
     OEMS_CUDA(cudaGetLastError());
     en->last_launches += 1;
   }
-  if (en->profiling) {
+  if (en->fus.use && (en->profiling || (en->flags & OEMS_ENGINE_NO_GRAPHS))) {
+    if (en->profiling && en->prof_ev.empty()) {
+      en->prof_ev.resize(256, nullptr);
+      for (auto& e : en->prof_ev) OEMS_CUDA(cudaEventCreate(&e));
+    }
+    OEMS_TRY(launch_steps_fused(en, steps));
+  } else if (en->profiling) {
     OEMS_TRY(launch_steps_profiled(en, steps));
   } else if (en->flags & OEMS_ENGINE_NO_GRAPHS) {
     OEMS_TRY(launch_steps_direct(en, steps));
@@ -1461,7 +1541,7 @@ static oems_status run_span(oems_engine* en, long long base, int steps) {
     OEMS_TRY(get_graph(en, steps, &exec));
     OEMS_CUDA(cudaGraphLaunch(exec, en->stream));
   }
-  en->last_launches += (uint64_t)steps * kernels_per_step(en);
+  en->last_launches += en->fus.use ? fused_launches(en, steps) : (uint64_t)steps * kernels_per_step(en);
   return OEMS_OK;
 }
 
@@ -1928,6 +2008,10 @@ static oems_status create(const oems_operator_desc* d, oems_engine** out) {
   return OEMS_OK;
 }
 
+}  // namespace oems
+#include "fused_host.cuh"
+namespace oems {
+
 static oems_status upload_excitations(oems_engine* en, const oems_batch* b) {
   en->nexc = (int)b->num_excitations;
   if (en->nexc == 0) return OEMS_OK;
@@ -1966,7 +2050,7 @@ static oems_status upload_excitations(oems_engine* en, const oems_batch* b) {
                                 cudaMemcpyHostToDevice, en->stream));
   // the host buffers are borrowed only for this call
   OEMS_CUDA(cudaStreamSynchronize(en->stream));
-  return OEMS_OK;
+  return en->fus.use ? fused_upload_sources(en, b, off, cnt) : OEMS_OK;
 }
 
 // Twiddles of the steps of the next batch: the sample after batch step s is
@@ -2013,7 +2097,15 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
   EngineScope guard(en);
   const auto t_start = std::chrono::steady_clock::now();
   en->last_launches = 0;
-  if (!en->tuned) OEMS_TRY(autotune(en));
+  bool fused = false;
+  OEMS_TRY(fused_ready(en, &fused));
+  if (fused != en->fus.use) en->graph_epoch++;
+  en->fus.use = fused;
+  if (fused) {
+    if (!en->fus.tuned) OEMS_TRY(fused_tune(en));
+  } else if (!en->tuned) {
+    OEMS_TRY(autotune(en));
+  }
   const int prev_nexc = en->nexc;
   OEMS_TRY(upload_excitations(en, b));
   if (prev_nexc != en->nexc) en->graph_epoch++;  // nexc is baked into captured graphs
@@ -2025,6 +2117,14 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
       OEMS_CUDA(en->d_traces.ensure(need));
       en->graph_epoch++;
     }
+  }
+  uint64_t span_cap = 1u << 20;
+  if (fused && nprobe > 0) {
+    span_cap = std::min(span_cap, fused_span_cap(en));
+    uint64_t longest = std::min(steps, span_cap);
+    if (b->sample_interval > 0) longest = std::min<uint64_t>(longest, b->sample_interval);
+    if (b->has_energy_decay_db && b->check_interval > 0) longest = std::min<uint64_t>(longest, b->check_interval + 1);
+    OEMS_TRY(fused_taps_ready(en, longest));
   }
   for (FieldDftHost& d : en->fdumps) OEMS_TRY(fill_twiddles(en, d.tab.get(), d.freqs, d.interval, steps));
   for (Nf2ffHost& x : en->boxes) OEMS_TRY(fill_twiddles(en, x.tab.get(), x.freqs, x.interval, steps));
@@ -2084,7 +2184,7 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
     }
     uint64_t span = steps - s;
     if (ev != UINT64_MAX && ev - cur + 1 < span) span = ev - cur + 1;
-    span = std::min<uint64_t>(span, 1u << 20);
+    span = std::min<uint64_t>(span, span_cap);
     OEMS_TRY(run_span(en, (long long)s, (int)span));
     s += span;
     executed = s;
@@ -2402,6 +2502,7 @@ static oems_status add_cpml(oems_engine* en, const oems_cpml_desc* d) {
   en->cpml.on = true;
   en->cpml.desc = *d;
   en->tuned = false;  // the CPML kernels get their own launch shape
+  en->fus.tuned = false;
   LaunchShape s = en->shape;
   OEMS_TRY(size_grid(en, s));
   apply_shape(en, s);
@@ -3647,6 +3748,17 @@ oems_status oems_engine_set_kernel_profiling(oems_engine* engine, int32_t enable
 oems_status oems_engine_launch_info(const oems_engine* engine, int32_t* staged, int32_t* threads, int32_t* ichunk,
                                     int32_t* rows_per_tile, int32_t* stages, int32_t* grid) {
   if (!engine) return fail(OEMS_ERR_INVALID_ARGUMENT, "NULL engine");
+  if (engine->fus.use) {
+    const FusedPlan& p = engine->fus.plan[fused_max_steps(engine) - 1];
+    const FusedBox& B = p.box[p.nbox - 1];
+    if (staged) *staged = 5;
+    if (threads) *threads = p.nt[p.items[0] ? 0 : 1];
+    if (ichunk) *ichunk = B.xlen;
+    if (rows_per_tile) *rows_per_tile = B.ty;
+    if (stages) *stages = p.steps;
+    if (grid) *grid = p.items[0] + p.items[1];
+    return OEMS_OK;
+  }
   const LaunchShape& s = engine->shape;
   if (staged) *staged = shape_kind(s);
   if (threads) *threads = s.tma ? s.nconsumer + 32 : s.block;

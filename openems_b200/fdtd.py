@@ -1051,7 +1051,8 @@ class Engine:
     def __init__(self, operator: Operator, engine_type: EngineType = EngineType.Cuda, *,
                  device: int = -1, compressed: bool = False, autotune: bool = True,
                  graphs: bool = True, kernels: str = "auto", storage: str = "f32"):
-        """kernels: "auto" (tuner picks), "register", "staged" (bulk-async),
+        """kernels: "auto" (fused one- and two-step passes where they apply,
+        else the tuner picks), "register", "staged" (bulk-async),
         "split" (staged between the x / y CPML slabs, register on them) or
         "zsplit" (plain register kernels on the CPML-free box, CPML register
         kernels on every slab cell) or "pipe" (pipelined register kernels:
@@ -1338,8 +1339,10 @@ class Engine:
     def tune_report(self) -> list:
         """Launch shapes the autotuner timed for this grid: dicts with kind (0
         register, 1 staged, 2 staged interior + register slabs, 3 register
-        z-only interior + full-CPML slabs), threads, ichunk, extra (stages or
-        prefetch distance), reps and ms (device time of the timed H + E pairs)."""
+        z-only interior + full-CPML slabs, 5 fused passes), threads, ichunk,
+        extra (stages or prefetch distance; fused: 1000 boxes + 10 chunks a
+        tile + steps a pass), reps and ms (device time of the timed H + E
+        pairs; fused: of `reps` steps)."""
         n = N.c_u64()
         N.check(N.lib().oems_engine_tune_report(self._h, None, 0, ctypes.byref(n)))
         rec = np.zeros(int(n.value), dtype=[("kind", "<i4"), ("threads", "<i4"), ("ichunk", "<i4"),

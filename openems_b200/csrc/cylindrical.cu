@@ -22,6 +22,9 @@
 
 namespace oems {
 extern thread_local std::string g_last_error;
+// pipelined copy of device arrays to pageable memory (engine.cu)
+cudaError_t copy_out(int device, float* const* dst, const float* const* src, int count, size_t rows, size_t width,
+                     size_t pitch, cudaStream_t after);
 }
 
 struct oems_cyl_engine {
@@ -260,13 +263,17 @@ static oems_status cyl_copy(oems_cyl_engine* en, float* const* host6, bool to_ho
   if (!en || !host6) return cfail(OEMS_ERR_INVALID_ARGUMENT, "NULL argument");
   Dev g(en->device);
   const size_t bytes = (size_t)en->n * sizeof(float);
-  for (int c = 0; c < 6; ++c) {
+  for (int c = 0; c < 6; ++c)
     if (!host6[c]) return cfail(OEMS_ERR_INVALID_ARGUMENT, "field pointer is NULL");
-    if (to_host)
-      CYL_CUDA(cudaMemcpyAsync(host6[c], en->at(c), bytes, cudaMemcpyDeviceToHost, en->stream));
-    else
-      CYL_CUDA(cudaMemcpyAsync(en->at(c), host6[c], bytes, cudaMemcpyHostToDevice, en->stream));
+  if (to_host) {
+    const float* src[6];
+    for (int c = 0; c < 6; ++c) src[c] = en->at(c);
+    const size_t nz = (size_t)en->nz;
+    CYL_CUDA(oems::copy_out(en->device, host6, src, 6, (size_t)en->n / nz, nz, nz, en->stream));
+    return OEMS_OK;
   }
+  for (int c = 0; c < 6; ++c)
+    CYL_CUDA(cudaMemcpyAsync(en->at(c), host6[c], bytes, cudaMemcpyHostToDevice, en->stream));
   CYL_CUDA(cudaStreamSynchronize(en->stream));
   return OEMS_OK;
 }

@@ -582,7 +582,7 @@ struct FusedKey {
 struct FusedHost {
   int state = 0;      // 0 not looked at, 1 prepared, -1 not for this engine
   bool use = false;   // this batch runs as fused passes
-  bool tuned = false;
+  bool tuned = false, tuned_pack = false;
   int parity = 0;     // which of the two buffer sets is current
   DevBuf<char> alt;   // the buffers the next pass writes
   DevBuf<float> psi;
@@ -591,7 +591,11 @@ struct FusedHost {
   int id_bytes = 0, ntable = 0;
   DevBuf<uint8_t> own_ids;
   DevBuf<float> own_table;
-  FusedPlan plan[2];
+  FusedPlan plan[2];       // passes of one and two steps, alone on the device
+  FusedPlan pack_plan[2];  // ... as one of a pack's engines
+  int pack_sms = 0;        // SMs' worth of work pack_plan was made for
+  bool packed = false;     // the pack's plans are in use
+  const FusedPlan& current(int steps) const { return packed ? pack_plan[steps - 1] : plan[steps - 1]; }
   DevBuf<int> src_i;         // plane offsets, keys, element / direction / kind
   DevBuf<long long> src_q;   // first sample and sample count
   int src_lo = 0, src_hi = 0;
@@ -2102,8 +2106,9 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
   en->last_launches = 0;
   bool fused = false;
   OEMS_TRY(fused_ready(en, &fused));
-  if (fused != en->fus.use) en->graph_epoch++;
+  if (fused != en->fus.use || en->fus.packed) en->graph_epoch++;
   en->fus.use = fused;
+  en->fus.packed = false;
   if (fused) {
     if (!en->fus.tuned) OEMS_TRY(fused_tune(en));
   } else if (!en->tuned) {
@@ -2122,13 +2127,7 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
     }
   }
   uint64_t span_cap = 1u << 20;
-  if (fused && nprobe > 0) {
-    span_cap = std::min(span_cap, fused_span_cap(en));
-    uint64_t longest = std::min(steps, span_cap);
-    if (b->sample_interval > 0) longest = std::min<uint64_t>(longest, b->sample_interval);
-    if (b->has_energy_decay_db && b->check_interval > 0) longest = std::min<uint64_t>(longest, b->check_interval + 1);
-    OEMS_TRY(fused_taps_ready(en, longest));
-  }
+  if (fused) OEMS_TRY(fused_spans(en, b, &span_cap));
   for (FieldDftHost& d : en->fdumps) OEMS_TRY(fill_twiddles(en, d.tab.get(), d.freqs, d.interval, steps));
   for (Nf2ffHost& x : en->boxes) OEMS_TRY(fill_twiddles(en, x.tab.get(), x.freqs, x.interval, steps));
   // TF/SF: this batch's 1D-grid values; the state is kept to replay a batch
@@ -2673,7 +2672,7 @@ static oems_status add_cpml(oems_engine* en, const oems_cpml_desc* d) {
   en->cpml.on = true;
   en->cpml.desc = *d;
   en->tuned = false;  // the CPML kernels get their own launch shape
-  en->fus.tuned = false;
+  en->fus.tuned = en->fus.tuned_pack = false;
   LaunchShape s = en->shape;
   OEMS_TRY(size_grid(en, s));
   apply_shape(en, s);
@@ -3920,7 +3919,7 @@ oems_status oems_engine_launch_info(const oems_engine* engine, int32_t* staged, 
                                     int32_t* rows_per_tile, int32_t* stages, int32_t* grid) {
   if (!engine) return fail(OEMS_ERR_INVALID_ARGUMENT, "NULL engine");
   if (engine->fus.use) {
-    const FusedPlan& p = engine->fus.plan[fused_max_steps(engine) - 1];
+    const FusedPlan& p = engine->fus.current(fused_max_steps(engine));
     const FusedBox& B = p.box[p.nbox - 1];
     if (staged) *staged = 5;
     if (threads) *threads = p.nt[p.items[0] ? 0 : 1];
@@ -4341,6 +4340,33 @@ static oems_status pack_run_span(oems_pack* p, long long base, int steps) {
   return OEMS_OK;
 }
 
+// Pinned room for the energies of n engines.
+static oems_status pack_host_energy(oems_pack* p, size_t n) {
+  if (p->h_energy_cap < n) {
+    pinned_put(p->h_energy, p->h_energy_cap * 2 * sizeof(double));
+    p->h_energy = nullptr;
+    p->h_energy_cap = 0;
+    void* q = nullptr;
+    OEMS_CUDA(pinned_get(&q, n * 2 * sizeof(double)));
+    p->h_energy = static_cast<double*>(q);
+    p->h_energy_cap = n;
+  }
+  return OEMS_OK;
+}
+
+// Energies of the active engines, each on its own stream, into
+// p->h_energy[2 k], [2 k + 1].
+static oems_status pack_energy_fused(oems_pack* p) {
+  for (size_t k = 0; k < p->active.size(); ++k) {
+    oems_engine* en = p->en[p->active[k]];
+    OEMS_TRY(launch_energy(en, en->d_energy.p));
+    OEMS_CUDA(cudaMemcpyAsync(p->h_energy + 2 * k, en->d_energy.p, 2 * sizeof(double), cudaMemcpyDeviceToHost,
+                              en->stream));
+  }
+  for (int i : p->active) OEMS_CUDA(cudaStreamSynchronize(p->en[i]->stream));
+  return OEMS_OK;
+}
+
 // Energies of the active engines into p->h_energy[2 k], [2 k + 1].
 static oems_status pack_energy(oems_pack* p) {
   const int na = (int)p->active.size();
@@ -4355,15 +4381,7 @@ static oems_status pack_energy(oems_pack* p) {
   const float hs = p->en[p->active[0]]->h_scale;
   k_energy_final_pack<<<na, 32, 0, p->stream>>>(p->energy.p, p->d_energy.p, 1.0 / ((double)hs * hs));
   OEMS_CUDA(cudaGetLastError());
-  if (p->h_energy_cap < (size_t)na) {
-    pinned_put(p->h_energy, p->h_energy_cap * 2 * sizeof(double));
-    p->h_energy = nullptr;
-    p->h_energy_cap = 0;
-    void* q = nullptr;
-    OEMS_CUDA(pinned_get(&q, (size_t)na * 2 * sizeof(double)));
-    p->h_energy = static_cast<double*>(q);
-    p->h_energy_cap = na;
-  }
+  OEMS_TRY(pack_host_energy(p, na));
   OEMS_CUDA(cudaMemcpyAsync(p->h_energy, p->d_energy.p, (size_t)na * 2 * sizeof(double), cudaMemcpyDeviceToHost,
                             p->stream));
   OEMS_CUDA(cudaStreamSynchronize(p->stream));
@@ -4380,6 +4398,36 @@ struct PackRun {
   std::vector<oems_energy_sample> samples;
   size_t peaked = 0;
 };
+
+// Whether every engine of the batch can run as fused passes; then the pack
+// launches each engine's own passes on the engine's stream (they share no
+// data), and the device runs as many of them side by side as fit.
+static oems_status pack_fused(oems_pack* p, const std::vector<int>& part, bool* yes) {
+  *yes = false;
+  if (p->shape_set) return OEMS_OK;  // a shape of the shared launches was asked for
+  int sms = 0;
+  OEMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
+  double cells = 0;
+  for (int i : part) {
+    EngineScope guard(p->en[i]);
+    bool ok = false;
+    OEMS_TRY(fused_ready(p->en[i], &ok));
+    if (!ok) return OEMS_OK;
+    cells += (double)p->en[i]->ncells_padded;
+  }
+  for (int i : part) {
+    oems_engine* en = p->en[i];
+    EngineScope guard(en);
+    // shapes for the engine's share of the device: with the others filling
+    // the rest, long x-runs and full tiles beat many short items
+    const int share = std::max(1, std::min(sms, (int)std::lround(sms * (double)en->ncells_padded / cells)));
+    OEMS_TRY(fused_pack_tune(en, share));
+    if (!en->fus.use || !en->fus.packed) en->graph_epoch++;
+    en->fus.use = en->fus.packed = true;
+  }
+  *yes = true;
+  return OEMS_OK;
+}
 
 static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches, oems_batch_result* results,
                                   oems_status* statuses) {
@@ -4401,6 +4449,9 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
   }
   if (part.empty()) return OEMS_OK;
   const uint64_t steps = b0->num_steps;
+  bool fused = false;
+  OEMS_TRY(pack_fused(p, part, &fused));
+  uint64_t span_cap = 1u << 20;
   for (int i : part) {
     oems_engine* en = p->en[i];
     EngineScope guard(en);
@@ -4409,19 +4460,31 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
     r.t0 = en->timestep;
     r.peak = r.b->initial_peak_energy;
     r.running = true;
+    const int prev_nexc = en->nexc;
     OEMS_TRY(upload_excitations(en, r.b));
-    const int np = en->nprobe();
-    if (np > 0) OEMS_CUDA(en->d_traces.ensure((size_t)std::max<uint64_t>(steps, 1) * np));
+    if (prev_nexc != en->nexc) en->graph_epoch++;
+    const size_t need = (size_t)std::max<uint64_t>(steps, 1) * en->nprobe();
+    if (en->nprobe() > 0 && en->d_traces.n < need) {
+      OEMS_CUDA(en->d_traces.ensure(need));
+      en->graph_epoch++;
+    }
+    if (fused) OEMS_TRY(fused_spans(en, r.b, &span_cap));
+    OEMS_CUDA(en->d_energy.ensure(2));
     OEMS_CUDA(cudaStreamSynchronize(en->stream));
   }
   DeviceGuard dg(p->device);
-  OEMS_TRY(pack_layout(p, part));
+  if (fused) {
+    p->active = part;
+    OEMS_TRY(pack_host_energy(p, part.size()));
+  } else {
+    OEMS_TRY(pack_layout(p, part));
+  }
   // tuned on the first batch, and again when the engines in the batch hold
   // under half the cells the shape was tuned on (a sweep's pack shrinks as
   // its instances end)
   double cells = 0;
   for (int i : part) cells += (double)p->en[i]->nx * p->en[i]->ny * p->en[i]->nz;
-  if (!p->shape_set && (!p->tuned || cells < 0.5 * p->tuned_cells)) OEMS_TRY(pack_tune(p));
+  if (!fused && !p->shape_set && (!p->tuned || cells < 0.5 * p->tuned_cells)) OEMS_TRY(pack_tune(p));
   const uint64_t si = b0->sample_interval, ci = b0->check_interval;
   const bool has_decay = b0->has_energy_decay_db != 0;
   const uint64_t t0 = R[part[0]].t0;
@@ -4438,14 +4501,24 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
     }
     uint64_t span = steps - s;
     if (ev != UINT64_MAX && ev - cur + 1 < span) span = ev - cur + 1;
-    span = std::min<uint64_t>(span, 1u << 20);
-    OEMS_TRY(pack_run_span(p, (long long)s, (int)span));
+    span = std::min<uint64_t>(span, span_cap);
+    if (fused) {
+      for (int i : p->active) {
+        EngineScope guard(p->en[i]);
+        OEMS_TRY(run_span(p->en[i], (long long)s, (int)span));
+      }
+    } else {
+      OEMS_TRY(pack_run_span(p, (long long)s, (int)span));
+    }
     s += span;
     const uint64_t last = t0 + s - 1;
     const bool do_sample = si > 0 && last % si == 0;
     const bool do_check = has_decay && ci > 0 && last > 0 && last % ci == 0;
     if (!do_sample && !do_check) continue;
-    OEMS_TRY(pack_energy(p));
+    if (fused)
+      OEMS_TRY(pack_energy_fused(p));
+    else
+      OEMS_TRY(pack_energy(p));
     std::vector<int> still;
     for (size_t k = 0; k < p->active.size(); ++k) {
       const int i = p->active[k];
@@ -4482,13 +4555,17 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
       }
     }
     if (still.size() != p->active.size()) {
-      if (still.empty())
-        p->active.clear();
+      if (still.empty() || fused)
+        p->active = still;
       else
         OEMS_TRY(pack_layout(p, still));
     }
   }
   for (int i : p->active) R[i].executed = s;
+  if (fused) {
+    for (int i : part) OEMS_CUDA(cudaStreamSynchronize(p->en[i]->stream));
+    p->active.clear();  // the shared launches' tables are not these engines'
+  }
   // probe DFTs of each engine's executed steps
   for (int i : part) {
     oems_engine* en = p->en[i];

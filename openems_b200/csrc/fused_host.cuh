@@ -557,6 +557,41 @@ static oems_status fused_tune(oems_engine* en) {
   return OEMS_OK;
 }
 
+// Shapes for an engine that shares the device with others: the model's best
+// on `sms` SMs.
+static oems_status fused_pack_tune(oems_engine* en, int sms) {
+  FusedHost& F = en->fus;
+  if (F.pack_sms == sms && F.tuned_pack) return OEMS_OK;
+  int smem_cta = 0, smem_sm = 0;
+  OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
+  OEMS_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, en->device));
+  for (int steps = 1; steps <= 2; ++steps) {
+    for (bool cpml : {false, true})
+      OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
+    const std::vector<FusedPlan> c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
+    if (c.empty()) return fail(OEMS_ERR_CUDA, "no tile shape of the fused kernels fits this device");
+    F.pack_plan[steps - 1] = c[0];
+  }
+  F.pack_sms = sms;
+  F.tuned_pack = true;
+  en->graph_epoch++;
+  return OEMS_OK;
+}
+
+// Longest spans of a batch, and the tap buffers for them.
+static oems_status fused_taps_ready(oems_engine* en, uint64_t span);
+static uint64_t fused_span_cap(const oems_engine* en);
+static oems_status fused_spans(oems_engine* en, const oems_batch* b, uint64_t* cap) {
+  if (en->nprobe() == 0) return OEMS_OK;
+  *cap = std::min(*cap, fused_span_cap(en));
+  uint64_t longest = std::min(b->num_steps, *cap);
+  if (b->sample_interval > 0) longest = std::min<uint64_t>(longest, b->sample_interval);
+  // (the first check comes after step check_interval, not after step 0)
+  if (b->has_energy_decay_db && b->check_interval > 0) longest = std::min<uint64_t>(longest, b->check_interval + 1);
+  return fused_taps_ready(en, longest);
+}
+
 // Sources of the batch sorted by (plane, row, chunk); equal cells keep the
 // list's order, which is the order they are applied in.
 static oems_status fused_upload_sources(oems_engine* en, const oems_batch* b, const std::vector<long long>& first,
@@ -670,7 +705,7 @@ static oems_status launch_steps_fused(oems_engine* en, int steps) {
     const int k = std::min(most, steps - s);
     if (hooks) OEMS_CUDA(launch_pre_e(en));
     if (ev) OEMS_CUDA(cudaEventRecord(ev[0], en->stream));
-    OEMS_CUDA(launch_fused(en, F.plan[k - 1], s, !hooks));
+    OEMS_CUDA(launch_fused(en, F.current(k), s, !hooks));
     if (ev) OEMS_CUDA(cudaEventRecord(ev[1], en->stream));
     fused_swap(en);
     if (hooks) {
@@ -695,7 +730,7 @@ static oems_status launch_steps_fused(oems_engine* en, int steps) {
 static uint64_t fused_launches(const oems_engine* en, int steps) {
   const int most = fused_max_steps(en);
   const uint64_t passes = (uint64_t)(steps + most - 1) / most;
-  const FusedPlan& p = en->fus.plan[most - 1];
+  const FusedPlan& p = en->fus.current(most);
   const uint64_t fd = en->fdumps.size() + en->boxes.size(), per = (p.items[0] ? 1 : 0) + (p.items[1] ? 1 : 0);
   if (fused_hooks(en)) return passes * (per + ext_kernels(en) + post_kernels(en));
   return passes * (per + fd) + (en->nprobe() > 0 ? 1 : 0);

@@ -391,7 +391,7 @@ static cudaError_t device_pool(int dev, bool create, cudaMemPool_t* out) {
 }
 
 // `bytes` of device memory ordered on stream s (the current device's pool).
-static cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;

@@ -4,8 +4,10 @@
 //
 // A and B are bf16, K-major (row-major with the reduction along the row),
 // row pitches multiples of 8 elements, K a multiple of 8; M and N are free.
-// A persistent grid (one CTA per SM) walks the 128 x BN output tiles; each
-// CTA is warp-specialised:
+// A persistent grid (one CTA per SM) walks the 128 x BN output tiles (or,
+// where there are too few for the SMs and K is long, parts of their K ranges,
+// each into its own f32 partial; k_gemm_sum adds those in order); each CTA is
+// warp-specialised:
 //   warp 0      one thread issues the TMA tile loads (cp.async.bulk.tensor,
 //               128-byte swizzle, zero fill past the matrix edge) of 64-wide
 //               K-blocks into a ring of shared-memory stages, each completed
@@ -126,7 +128,25 @@ struct GemmArgs {
   int M, N, K;
   float beta;
   int* err;
+  // splits > 1: item t is part t % splits (kb_per K-blocks) of tile t / splits,
+  // written to part + (t % splits) M N
+  int splits, kb_per;
+  float* part;
 };
+
+// C = sum of the parts, in order (+ beta C) (+ bias)
+__global__ void k_gemm_sum(const GemmArgs p) {
+  const long long n = (long long)p.M * p.N;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    float v = 0.f;
+    for (int s = 0; s < p.splits; ++s) v += __ldg(p.part + s * n + i);
+    const long long r = i / p.N;
+    const int c = (int)(i - r * p.N);
+    if (p.bias) v += __ldg(p.bias + c);
+    float* o = p.c + r * p.ldc + c;
+    *o = p.beta != 0.0f ? v + p.beta * *o : v;
+  }
+}
 
 template <int BN>
 struct GemmCfg {
@@ -151,7 +171,7 @@ __global__ void __launch_bounds__(192, 1)
   uint64_t* acc_empty = acc_full + 2;  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tn = (p.N + BN - 1) / BN, tiles = ((p.M + BM - 1) / BM) * tn;
+  const int tn = (p.N + BN - 1) / BN, tiles = ((p.M + BM - 1) / BM) * tn * p.splits;
   const int nkb = (p.K + BK - 1) / BK;
   const uint32_t sbase = tc::smem_u32(base);
 
@@ -185,8 +205,9 @@ __global__ void __launch_bounds__(192, 1)
     int it = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-      const int m0 = (t / tn) * BM, n0 = (t % tn) * BN;
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
+      const int tile = t / p.splits, k0 = (t % p.splits) * p.kb_per, k1 = min(k0 + p.kb_per, nkb);
+      const int m0 = (tile / tn) * BM, n0 = (tile % tn) * BN;
+      for (int kb = k0; kb < k1; ++kb, ++it) {
         const int st = it % S;
         if (!tc::mbar_wait(empty + st, (uint32_t)(((it / S) & 1) ^ 1), p.err)) {
           ok = false;
@@ -215,7 +236,8 @@ __global__ void __launch_bounds__(192, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem + (uint32_t)(b * BN);
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
+      const int k0 = (t % p.splits) * p.kb_per, k1 = min(k0 + p.kb_per, nkb);
+      for (int kb = k0; kb < k1; ++kb, ++it) {
         const int st = it % S;
         if (!tc::mbar_wait(full + st, (uint32_t)((it / S) & 1), p.err)) {
           ok = false;
@@ -228,7 +250,7 @@ __global__ void __launch_bounds__(192, 1)
           // K = 16 bf16 = 32 bytes further along the swizzled row
           const uint64_t ad = tc::sw128_desc(a_addr + k * 32);
           const uint64_t bd = tc::sw128_desc(b_addr + k * 32);
-          const uint32_t accum = (kb > 0 || k > 0) ? 1u : 0u;
+          const uint32_t accum = (kb > k0 || k > 0) ? 1u : 0u;
           asm volatile(
               "{\n\t.reg .pred p;\n\t"
               "setp.ne.b32 p, %4, 0;\n\t"
@@ -252,7 +274,10 @@ __global__ void __launch_bounds__(192, 1)
   } else if (warp >= 2) {
     // ---- epilogue: warp w reads accumulator lanes 32 (w % 4) .. + 31
     const int q = warp & 3;
-    const bool vec = (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0);
+    const bool split = p.splits > 1;
+    const int ldc = split ? p.N : p.ldc;
+    const float* bias = split ? nullptr : p.bias;
+    const float beta = split ? 0.0f : p.beta;
     int tl = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tl) {
       const int b = tl & 1;
@@ -260,7 +285,9 @@ __global__ void __launch_bounds__(192, 1)
       if (lane == 0) fine = tc::mbar_wait(acc_full + b, (uint32_t)((tl >> 1) & 1), p.err) ? 1 : 0;
       if (!__shfl_sync(0xffffffffu, fine, 0)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const int m0 = (t / tn) * BM, n0 = (t % tn) * BN;
+      const int tile = t / p.splits, m0 = (tile / tn) * BM, n0 = (tile % tn) * BN;
+      float* c = split ? p.part + (size_t)(t % p.splits) * p.M * p.N : p.c;
+      const bool vec = (ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(c) & 15) == 0);
       const int row = m0 + q * 32 + lane;
       for (int c0 = 0; c0 < BN && n0 + c0 < p.N; c0 += 32) {
         uint32_t v[32];
@@ -277,7 +304,7 @@ __global__ void __launch_bounds__(192, 1)
             : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (row < p.M) {
-          float* crow = p.c + (size_t)row * p.ldc;
+          float* crow = c + (size_t)row * ldc;
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const int col = n0 + c0 + e;
@@ -285,16 +312,16 @@ __global__ void __launch_bounds__(192, 1)
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               x[u] = __uint_as_float(v[e + u]);
-              if (p.bias && col + u < p.N) x[u] += __ldg(p.bias + col + u);
+              if (bias && col + u < p.N) x[u] += __ldg(bias + col + u);
             }
             if (vec && col + 3 < p.N) {
               float4* cp = reinterpret_cast<float4*>(crow + col);
-              if (p.beta != 0.0f) {
+              if (beta != 0.0f) {
                 const float4 o = *cp;
-                x[0] += p.beta * o.x;
-                x[1] += p.beta * o.y;
-                x[2] += p.beta * o.z;
-                x[3] += p.beta * o.w;
+                x[0] += beta * o.x;
+                x[1] += beta * o.y;
+                x[2] += beta * o.z;
+                x[3] += beta * o.w;
               }
               *cp = make_float4(x[0], x[1], x[2], x[3]);
             } else {
@@ -302,7 +329,7 @@ __global__ void __launch_bounds__(192, 1)
               for (int u = 0; u < 4; ++u) {
                 if (col + u >= p.N) break;
                 float* cp = crow + col + u;
-                *cp = p.beta != 0.0f ? x[u] + p.beta * *cp : x[u];
+                *cp = beta != 0.0f ? x[u] + beta * *cp : x[u];
               }
             }
           }

@@ -6,8 +6,9 @@
 // f32 accumulation; activations are kept as f32 (B, T, C) row-major with bf16
 // copies for the GEMM operands; weights are f32 masters with bf16 copies.
 // All entry points take device pointers and a CUDA stream (NULL = default)
-// and return an oems_status; nothing here allocates except the error word
-// (once per device, on first use).
+// and return an oems_status; what they allocate is the error word (once per
+// device) and, for split reductions, stream-ordered workspace from the
+// device's pool.
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -23,6 +24,9 @@
 
 namespace oems {
 extern thread_local std::string g_last_error;
+// stream-ordered memory of the current device's pool, kept for reuse until
+// oems_release_cached_memory (engine.cu)
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
 }
 
 namespace {
@@ -50,6 +54,21 @@ oems_status err_word(int** out) {
   }
   *out = g_err[dev];
   return OEMS_OK;
+}
+
+// Stream-ordered workspace of one call.
+struct Workspace {
+  void* p = nullptr;
+  cudaStream_t s;
+  explicit Workspace(void* stream) : s(reinterpret_cast<cudaStream_t>(stream)) {}
+  cudaError_t get(size_t bytes) { return oems::pool_alloc(&p, bytes, s); }
+  ~Workspace() {
+    if (p) cudaFreeAsync(p, s);
+  }
+};
+
+inline bool aligned16(const void* a, const void* b) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0;
 }
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }
@@ -121,6 +140,42 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* x, int ldx, __nv_bfloat16*
   }
 }
 
+__device__ __forceinline__ uint32_t bf16x2(float a, float b) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// The transpose for pitches and sizes that are multiples of 8: 64 x 64 tiles,
+// 16-byte loads and stores (the 2-byte form moves 64-byte rows at 1.4 TB/s;
+// 65536 x 640: 21 -> 9 us an average launch of the network's shapes).
+__global__ void __launch_bounds__(256) k_transpose_bf16_8(const __nv_bfloat16* x, int ldx, __nv_bfloat16* y, int ldy,
+                                                          int R, int C) {
+  __shared__ __nv_bfloat16 t[64][66];
+  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = (threadIdx.x >> 3) + 32 * h, c = (threadIdx.x & 7) * 8;
+    if (r0 + i < R && c0 + c < C) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + (size_t)(r0 + i) * ldx + c0 + c));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) *reinterpret_cast<uint32_t*>(&t[i][c + 2 * u]) = w[u];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = (threadIdx.x >> 3) + 32 * h, r = (threadIdx.x & 7) * 8;
+    if (c0 + c < C && r0 + r < R) {
+      uint32_t w[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        w[u] = (uint32_t)__bfloat16_as_ushort(t[r + 2 * u][c]) | (uint32_t)__bfloat16_as_ushort(t[r + 2 * u + 1][c]) << 16;
+      *reinterpret_cast<uint4*>(y + (size_t)(c0 + c) * ldy + r0 + r) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  }
+}
+
 // cols[(b, t), k * C + c] = x[b, t * s + k, c]  (bf16, row pitch ldc)
 __global__ void k_im2col(const float* x, __nv_bfloat16* cols, int B, int T, int C, int ks, int s, int Tout,
                          int ldc) {
@@ -175,6 +230,27 @@ __global__ void k_im2col_causal(const float* x, __nv_bfloat16* cols, int B, int 
   }
 }
 
+// The same for C and ldc multiples of 8 and 16-byte bases: 8 channels a
+// thread (two 16-byte loads, one 16-byte store, one division chain where the
+// general form has eight): 256 x 256 x 128 channels, 5 taps: 200 -> 25 us.
+__global__ void __launch_bounds__(256) k_im2col_causal8(const float* x, __nv_bfloat16* cols, long long rows, int T,
+                                                        int C, int ks, int dil, int ldc) {
+  const int per = ks * (C >> 3);  // 8-channel groups of a row
+  const long long n = rows * per;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long row = i / per;
+    const int g = (int)(i - row * per), k = g / (C >> 3), c = (g - k * (C >> 3)) * 8;
+    const int back = (ks - 1 - k) * dil, t = (int)(row % T);
+    uint4 o = make_uint4(0, 0, 0, 0);
+    if (t >= back) {
+      const float4* s = reinterpret_cast<const float4*>(x + (row - back) * C + c);
+      const float4 a = __ldg(s), b = __ldg(s + 1);
+      o = make_uint4(bf16x2(a.x, a.y), bf16x2(a.z, a.w), bf16x2(b.x, b.y), bf16x2(b.z, b.w));
+    }
+    *reinterpret_cast<uint4*>(cols + row * ldc + (long long)k * C + c) = o;
+  }
+}
+
 // Adjoint: dx[b, tau, c] = sum over k of dcols[(b, tau + (ks - 1 - k) dil), k C + c]
 // (terms past the end dropped), summed in k order.
 __global__ void k_col2im_causal(const float* dcols, int ldc, float* dx, int B, int T, int C, int ks, int dil) {
@@ -194,6 +270,28 @@ __global__ void k_col2im_causal(const float* dcols, int ldc, float* dx, int B, i
   }
 }
 
+// The same for C and ldc multiples of 4 and 16-byte bases, 4 channels a thread.
+__global__ void __launch_bounds__(256) k_col2im_causal4(const float* dcols, int ldc, float* dx, long long rows, int T,
+                                                        int C, int ks, int dil) {
+  const int per = C >> 2;
+  const long long n = rows * per;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long row = i / per;
+    const int c = (int)(i - row * per) * 4, tau = (int)(row % T);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = 0; k < ks; ++k) {
+      const int on = (ks - 1 - k) * dil;
+      if (tau + on >= T) continue;
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(dcols + (row + on) * ldc + (long long)k * C + c));
+      acc.x += v.x;
+      acc.y += v.y;
+      acc.z += v.z;
+      acc.w += v.w;
+    }
+    *reinterpret_cast<float4*>(dx + row * C + c) = acc;
+  }
+}
+
 // y = max(x, 0) in place, with a bf16 copy of y (pitch ldb, rows of width w)
 __global__ void k_relu(float* x, __nv_bfloat16* xb, long long rows, int w, int ldb) {
   const long long n = rows * w;
@@ -201,6 +299,19 @@ __global__ void k_relu(float* x, __nv_bfloat16* xb, long long rows, int w, int l
     const float v = fmaxf(x[i], 0.f);
     x[i] = v;
     if (xb) xb[(i / w) * ldb + i % w] = __float2bfloat16_rn(v);
+  }
+}
+
+// The same for widths and pitches that are multiples of 4, with a bf16 copy.
+__global__ void __launch_bounds__(256) k_relu4(float* x, __nv_bfloat16* xb, long long rows, int w, int ldb) {
+  const int per = w >> 2;
+  const long long n = rows * per;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    float4 v = reinterpret_cast<float4*>(x)[i];
+    v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+    reinterpret_cast<float4*>(x)[i] = v;
+    const long long row = i / per;
+    *reinterpret_cast<uint2*>(xb + row * ldb + (i - row * per) * 4) = make_uint2(bf16x2(v.x, v.y), bf16x2(v.z, v.w));
   }
 }
 
@@ -223,6 +334,61 @@ __global__ void k_colsum(const float* dy, long long rows, int w, float* db) {
     __syncthreads();
   }
   if (threadIdx.x == 0) db[c] = part[0];
+}
+
+// Long columns: block b sums rows [b per, b per + per) of every column into
+// part[b] (kV columns a thread, 32 row lanes, so rows are read whole and four
+// of a lane's are in flight); the second launch adds the parts, 8 lanes each
+// its own, in a fixed order.  65536 x 128: 37 us with a block per column.
+template <int kV>
+__global__ void __launch_bounds__(1024) k_colsum_part(const float* dy, long long rows, int w, long long per, float* part) {
+  __shared__ float red[32][32 * kV];
+  const int lane = threadIdx.x >> 5, q = threadIdx.x & 31;
+  const long long r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
+  for (int c0 = 0; c0 < w; c0 += 32 * kV) {
+    const int c = c0 + q * kV;
+    float acc[kV];
+#pragma unroll
+    for (int v = 0; v < kV; ++v) acc[v] = 0.f;
+    if (c < w) {
+#pragma unroll 4
+      for (long long r = r0 + lane; r < r1; r += 32) {
+        if constexpr (kV == 4) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(dy + r * w + c));
+          acc[0] += x.x;
+          acc[1] += x.y;
+          acc[2] += x.z;
+          acc[3] += x.w;
+        } else {
+          acc[0] += __ldg(dy + r * w + c);
+        }
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < kV; ++v) red[lane][q * kV + v] = acc[v];
+    __syncthreads();
+    for (int x = threadIdx.x; x < 32 * kV && c0 + x < w; x += blockDim.x) {
+      float sum = 0.f;
+#pragma unroll 8
+      for (int l = 0; l < 32; ++l) sum += red[l][x];
+      part[(long long)blockIdx.x * w + c0 + x] = sum;
+    }
+    __syncthreads();
+  }
+}
+__global__ void __launch_bounds__(256) k_colsum_add(const float* part, int parts, int w, float* db) {
+  __shared__ float red[8][32];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
+  float acc = 0.f;
+  if (c < w)
+#pragma unroll 4
+    for (int p = lane; p < parts; p += 8) acc += __ldg(part + (long long)p * w + c);
+  red[lane][threadIdx.x & 31] = acc;
+  __syncthreads();
+  if (lane == 0 && c < w) {
+    for (int l = 1; l < 8; ++l) acc += red[l][threadIdx.x];
+    db[c] = acc;
+  }
 }
 
 // g = 2 (p - t) w_row / n ; loss partials per block (sum of w_row (p - t)^2)
@@ -302,11 +468,38 @@ oems_status oems_tc_gemm_bf16(const void* a, int lda, const void* b, int ldb, fl
     const long long cost = waves * (cand + 64);
     if (best < 0 || cost < best) best = cost, BN = cand;
   }
+  // few tiles and a long K (the weight gradients: 128 x 640 outputs over K =
+  // 65,536 ran on 10 of 148 SMs, 215 us): the K range in parts of at least 8
+  // blocks, as many as the SMs take in one wave.  Fewer than half the SMs
+  // busy, or the sum of the parts costs more than it gives.
+  p.splits = 1;
+  p.kb_per = (K + 63) / 64;
+  if (tm * ((N + BN - 1) / BN) * 2 <= sms && p.kb_per >= 32) {
+    long long fewest = -1;
+    int split_bn = BN;
+    for (int cand : {256, 128, 64}) {
+      const long long t = tm * ((N + cand - 1) / cand);
+      const long long parts = std::max<long long>(1, std::min<long long>(sms / t, p.kb_per / 8));
+      const long long cost = ((p.kb_per + parts - 1) / parts) * (cand + 64);
+      if (t <= sms && (fewest < 0 || cost < fewest)) fewest = cost, split_bn = cand;
+    }
+    BN = split_bn;
+    const long long t = tm * ((N + BN - 1) / BN);
+    const int nkb = p.kb_per;
+    const int parts = (int)std::max<long long>(1, std::min<long long>(sms / t, nkb / 8));
+    p.kb_per = (nkb + parts - 1) / parts;
+    p.splits = (nkb + p.kb_per - 1) / p.kb_per;
+  }
+  Workspace ws(stream);
+  if (p.splits > 1) {
+    PK_CUDA(ws.get((size_t)p.splits * M * N * sizeof(float)));
+    p.part = static_cast<float*>(ws.p);
+  }
   CUtensorMap ta, tb;
   st = bf16_map(enc, &ta, a, lda, K, M, 128);
   if (st == OEMS_OK) st = bf16_map(enc, &tb, b, ldb, K, N, BN);
   if (st != OEMS_OK) return st;
-  const long long tiles = tm * ((N + BN - 1) / BN);
+  const long long tiles = tm * ((N + BN - 1) / BN) * p.splits;
   const int grid = (int)std::min<long long>(tiles, sms);
   if (BN == 256) {
     PK_CUDA(launch_gemm<256>(ta, tb, p, grid, stream));
@@ -315,6 +508,7 @@ oems_status oems_tc_gemm_bf16(const void* a, int lda, const void* b, int ldb, fl
   } else {
     PK_CUDA(launch_gemm<64>(ta, tb, p, grid, stream));
   }
+  if (p.splits > 1) oems::k_gemm_sum<<<grid_for((long long)M * N, 2048), 256, 0, S(stream)>>>(p);
   PK_CUDA(cudaGetLastError());
   return OEMS_OK;
 }
@@ -349,6 +543,15 @@ oems_status oems_pk_f32_to_bf16(const float* x, void* y, int64_t n, void* stream
 }
 
 oems_status oems_pk_transpose_bf16(const void* x, int ldx, void* y, int ldy, int R, int C, void* stream) {
+  if (R % 8 == 0 && C % 8 == 0 && ldx % 8 == 0 && ldy % 8 == 0 && aligned16(x, y)) {
+    const dim3 g8((C + 63) / 64, (R + 63) / 64);
+    if (g8.y <= 65535) {
+      k_transpose_bf16_8<<<g8, 256, 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(x), ldx,
+                                                    static_cast<__nv_bfloat16*>(y), ldy, R, C);
+      PK_CUDA(cudaGetLastError());
+      return OEMS_OK;
+    }
+  }
   const dim3 grid((C + 31) / 32, (R + 31) / 32);
   k_transpose_bf16<<<grid, dim3(32, 8), 0, S(stream)>>>(static_cast<const __nv_bfloat16*>(x), ldx,
                                                        static_cast<__nv_bfloat16*>(y), ldy, R, C);
@@ -377,6 +580,13 @@ oems_status oems_pk_col2im(const float* dcols, int ldc, float* dx, int B, int T,
 oems_status oems_pk_im2col_causal(const float* x, void* cols, int B, int T, int C, int ks, int dil, int ldc,
                                   void* stream) {
   if (ks < 1 || dil < 1 || ldc < ks * C) return pfail(OEMS_ERR_CONFIG, "im2col_causal: bad kernel, dilation or pitch");
+  if (C % 8 == 0 && ldc % 8 == 0 && aligned16(x, cols)) {
+    const long long rows = (long long)B * T;
+    k_im2col_causal8<<<grid_for(rows * ks * (C / 8), 148 * 16), 256, 0, S(stream)>>>(
+        x, static_cast<__nv_bfloat16*>(cols), rows, T, C, ks, dil, ldc);
+    PK_CUDA(cudaGetLastError());
+    return OEMS_OK;
+  }
   const long long n = (long long)B * T * ks * C;
   k_im2col_causal<<<grid_for(n, 8192), 256, 0, S(stream)>>>(x, static_cast<__nv_bfloat16*>(cols), B, T, C, ks, dil,
                                                             ldc);
@@ -387,6 +597,12 @@ oems_status oems_pk_im2col_causal(const float* x, void* cols, int B, int T, int 
 oems_status oems_pk_col2im_causal(const float* dcols, int ldc, float* dx, int B, int T, int C, int ks, int dil,
                                   void* stream) {
   if (ks < 1 || dil < 1 || ldc < ks * C) return pfail(OEMS_ERR_CONFIG, "col2im_causal: bad kernel, dilation or pitch");
+  if (C % 4 == 0 && ldc % 4 == 0 && aligned16(dcols, dx)) {
+    const long long rows = (long long)B * T;
+    k_col2im_causal4<<<grid_for(rows * (C / 4), 148 * 16), 256, 0, S(stream)>>>(dcols, ldc, dx, rows, T, C, ks, dil);
+    PK_CUDA(cudaGetLastError());
+    return OEMS_OK;
+  }
   const long long n = (long long)B * T * C;
   k_col2im_causal<<<grid_for(n, 8192), 256, 0, S(stream)>>>(dcols, ldc, dx, B, T, C, ks, dil);
   PK_CUDA(cudaGetLastError());
@@ -394,6 +610,11 @@ oems_status oems_pk_col2im_causal(const float* dcols, int ldc, float* dx, int B,
 }
 
 oems_status oems_pk_relu(float* x, void* xb, int64_t rows, int w, int ldb, void* stream) {
+  if (xb && w % 4 == 0 && ldb % 4 == 0 && aligned16(x, xb)) {
+    k_relu4<<<grid_for(rows * (w / 4), 148 * 16), 256, 0, S(stream)>>>(x, static_cast<__nv_bfloat16*>(xb), rows, w, ldb);
+    PK_CUDA(cudaGetLastError());
+    return OEMS_OK;
+  }
   const long long n = rows * w;
   k_relu<<<grid_for(n, 8192), 256, 0, S(stream)>>>(x, static_cast<__nv_bfloat16*>(xb), rows, w, ldb);
   PK_CUDA(cudaGetLastError());
@@ -407,6 +628,20 @@ oems_status oems_pk_relu_bwd(float* dy, const float* y, int64_t n, void* stream)
 }
 
 oems_status oems_pk_colsum(const float* dy, int64_t rows, int w, float* db, void* stream) {
+  if (rows >= 4096) {
+    const int parts = 148;
+    const long long per = (rows + parts - 1) / parts;
+    Workspace ws(stream);
+    PK_CUDA(ws.get((size_t)parts * w * sizeof(float)));
+    float* part = static_cast<float*>(ws.p);
+    if (w % 4 == 0 && aligned16(dy, dy))
+      k_colsum_part<4><<<parts, 1024, 0, S(stream)>>>(dy, rows, w, per, part);
+    else
+      k_colsum_part<1><<<parts, 1024, 0, S(stream)>>>(dy, rows, w, per, part);
+    k_colsum_add<<<blocks(w, 32), 256, 0, S(stream)>>>(part, parts, w, db);
+    PK_CUDA(cudaGetLastError());
+    return OEMS_OK;
+  }
   k_colsum<<<w, 256, 0, S(stream)>>>(dy, rows, w, db);
   PK_CUDA(cudaGetLastError());
   return OEMS_OK;

@@ -53,8 +53,11 @@ oems_status cfail(oems_status st, const std::string& m) {
     if (e_ != cudaSuccess) return cfail(OEMS_ERR_CUDA, cudaGetErrorString(e_)); \
   } while (0)
 
-constexpr int kCylRowThreads = 128;  // z cells per block in the row form
-constexpr unsigned kCylRowMinZ = 128;  // shorter z rows use the flat form
+// Row form: blocks of 256 threads, a z part of a row (a multiple of 32 cells,
+// as even as the row divides) times as many rows as fill the block.  Blocks of
+// 128 cells of one row left 37% of the lanes idle at 160 cells a row.
+constexpr int kCylRowThreads = 256;
+constexpr unsigned kCylRowMinZ = 24;  // shorter z rows use the flat form
 
 struct CylArgs {
   float* e[3];
@@ -116,12 +119,13 @@ __global__ void __launch_bounds__(256) k_cyl_flat(const CylArgs a) {
   }
 }
 
-// Row form: blockIdx.y walks the (rho, alpha) rows, threads the z cells of
-// a row, so no per-cell division and every row access is coalesced.
+// Row form: blockIdx.y and threadIdx.y walk the (rho, alpha) rows, blockIdx.x
+// and threadIdx.x the z cells of a row, so no per-cell division and every row
+// access is coalesced.
 template <bool kVoltage>
 __global__ void __launch_bounds__(kCylRowThreads) k_cyl_rows(const CylArgs a) {
   const unsigned rows = a.nr * a.na;
-  for (unsigned row = blockIdx.y; row < rows; row += gridDim.y) {
+  for (unsigned row = blockIdx.y * blockDim.y + threadIdx.y; row < rows; row += gridDim.y * blockDim.y) {
     const unsigned i = row / a.na, j = row - i * a.na;
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < a.nz; k += gridDim.x * blockDim.x) {
       if (kVoltage)
@@ -228,17 +232,20 @@ static oems_status cyl_launch(oems_cyl_engine* en, uint64_t steps) {
   const CylArgs v = args(en, true), c = args(en, false);
   const int gn = grid_of(en->n), gr = grid_of(en->na * en->nz);
   const bool rows = (unsigned)en->nz >= kCylRowMinZ;
-  const long long nrows = en->nr * en->na, per = (nrows + 65534) / 65535;  // gridDim.y <= 65535
-  const dim3 grow((unsigned)((en->nz + kCylRowThreads - 1) / kCylRowThreads), (unsigned)((nrows + per - 1) / per));
+  const long long parts = (en->nz + kCylRowThreads - 1) / kCylRowThreads;
+  const long long bz = std::max<long long>(32, (((en->nz + parts - 1) / parts) + 31) / 32 * 32);
+  const dim3 brow((unsigned)bz, (unsigned)std::max<long long>(1, kCylRowThreads / bz));
+  const long long nrows = (en->nr * en->na + brow.y - 1) / brow.y, per = (nrows + 65534) / 65535;  // gridDim.y <= 65535
+  const dim3 grow((unsigned)((en->nz + bz - 1) / bz), (unsigned)((nrows + per - 1) / per));
   CYL_CUDA(cudaEventRecord(en->ev[0], en->stream));
   for (uint64_t s = 0; s < steps; ++s) {
     if (rows)
-      k_cyl_rows<true><<<grow, kCylRowThreads, 0, en->stream>>>(v);
+      k_cyl_rows<true><<<grow, brow, 0, en->stream>>>(v);
     else
       k_cyl_flat<true><<<gn, 256, 0, en->stream>>>(v);
     if (en->r0) k_cyl_r0<<<gr, 256, 0, en->stream>>>(v);
     if (rows)
-      k_cyl_rows<false><<<grow, kCylRowThreads, 0, en->stream>>>(c);
+      k_cyl_rows<false><<<grow, brow, 0, en->stream>>>(c);
     else
       k_cyl_flat<false><<<gn, 256, 0, en->stream>>>(c);
     en->timestep += 1;

@@ -305,7 +305,7 @@ static double fused_item_cost(const FusedPlan& p, int b, int planes, const int (
   const int c = b < p.ncpml ? 1 : 0;
   const double w = p.box[b].axes == 7 ? 2.2 : p.box[b].axes == 6 ? 1.8 : p.box[b].axes == 4 ? 1.7 : 1.0;
   const double slots = (p.steps == 2 ? 5.5 : 2.8) * w * occ[c] * p.nt[c], latency = (p.steps == 2 ? 1800.0 : 1000.0) * w;
-  return (planes + p.steps + 3) * std::max(latency, slots) / occ[c];
+  return (planes + (p.steps == 2 ? 4.5 : 2.5)) * std::max(latency, slots) / occ[c];
 }
 
 static double fused_cost(const FusedPlan& p, int sms, const int (&occ)[2], std::vector<double>& heap) {
@@ -323,6 +323,12 @@ static double fused_cost(const FusedPlan& p, int sms, const int (&occ)[2], std::
   }
   return *std::max_element(heap.begin(), heap.end());
 }
+
+// Grids below this many cells are tuned over more shapes: a pass takes tens
+// of microseconds, and latency the model does not see decides.  (One-step
+// passes, with fewer planes of lead-in, measure level with two-step ones there
+// when launched back to back, and a fifth slower inside a graph.)
+constexpr long long kFusedSmall = 3000000;
 
 // Shapes for passes of `steps`, best first by the model.
 static std::vector<FusedPlan> fused_shapes(const oems_engine* en, int steps, int sms, size_t smem_cta,
@@ -368,8 +374,7 @@ static std::vector<FusedPlan> fused_shapes(const oems_engine* en, int steps, int
     if (!ok) continue;
     const FusedBox& last = p.box[p.nbox - 1];
     const int planes = last.i1 - last.i0;
-    FusedPlan first, second;
-    first.cost = second.cost = 1e30;
+    std::vector<FusedPlan> kept;  // the best x-runs of this CTA size
     for (int n = 1, prev = 0; n <= planes; n += 1 + n / 8) {
       const int len = (planes + n - 1) / n;
       if (len == prev) continue;
@@ -393,15 +398,12 @@ static std::vector<FusedPlan> fused_shapes(const oems_engine* en, int steps, int
       }
       if (p.items[0] + p.items[1] > 16 * sms) break;
       p.cost = fused_cost(p, sms, occ, heap);
-      if (p.cost < first.cost) {
-        second = first;
-        first = p;
-      } else if (p.cost < second.cost) {
-        second = p;
-      }
+      kept.push_back(p);
     }
-    if (first.cost < 1e30) all.push_back(first);
-    if (second.cost < 1e30) all.push_back(second);
+    const size_t most = std::min<size_t>(kept.size(), en->ncells_padded < kFusedSmall ? 5 : 2);
+    std::partial_sort(kept.begin(), kept.begin() + most, kept.end(),
+                      [](const FusedPlan& x, const FusedPlan& y) { return x.cost < y.cost; });
+    all.insert(all.end(), kept.begin(), kept.begin() + most);
   }
   std::sort(all.begin(), all.end(), [](const FusedPlan& x, const FusedPlan& y) { return x.cost < y.cost; });
   return all;
@@ -452,6 +454,23 @@ static FusedArgs fused_args(oems_engine* en, int local, bool posts) {
   return a;
 }
 
+// A pass that is a single launch may start while the kernel before it in the
+// stream is draining: until its griddepcontrol.wait it only reads its
+// arguments, the table and the profiles.
+static void launch_pass(FusedKernel k, const FusedArgs& a, int grid, int nt, size_t smem, cudaStream_t s, bool early) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)nt);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&c, k, a);  // an error is seen by the caller's cudaGetLastError
+}
+
 // One pass of p.steps steps, starting at step `local` of the span: the boxes
 // with slabs on a second stream beside the others (they read and write the
 // same buffers, but no cell is written by both).
@@ -467,12 +486,12 @@ static cudaError_t launch_fused(oems_engine* en, const FusedPlan& p, int local, 
     a.nbox = p.ncpml;
     std::copy(p.box, p.box + p.ncpml, a.box);
     a.pairs = p.pairs;
-    pick_fused(en, p.steps, true)<<<p.items[1], p.nt[1], p.smem[1], side>>>(a);
+    launch_pass(pick_fused(en, p.steps, true), a, p.items[1], p.nt[1], p.smem[1], side, !fork);
   }
   if (p.items[0]) {
     a.nbox = p.nbox - p.ncpml;
     std::copy(p.box + p.ncpml, p.box + p.nbox, a.box);
-    pick_fused(en, p.steps, false)<<<p.items[0], p.nt[0], p.smem[0], en->stream>>>(a);
+    launch_pass(pick_fused(en, p.steps, false), a, p.items[0], p.nt[0], p.smem[0], en->stream, !p.items[1]);
   }
   if (fork) {
     cudaEventRecord(en->join_ev, side);
@@ -518,14 +537,15 @@ static oems_status fused_tune(oems_engine* en) {
       c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
     if (c.empty()) return fail(OEMS_ERR_CUDA, "no tile shape of the fused kernels fits this device");
     // one-step passes only finish odd spans unless an extension needs them
-    const size_t most = cached || !time_it ? 1 : steps == fused_max_steps(en) ? 12 : 3;
+    const bool small = en->ncells_padded < kFusedSmall;
+    const size_t most = cached || !time_it ? 1 : steps != fused_max_steps(en) ? 3 : small ? 30 : 12;
     if (c.size() > most) c.resize(most);
     FusedPlan best = c[0];
     if (c.size() > 1) {
       float best_ms = 1e30f;
       for (FusedPlan& p : c) {
         OEMS_CUDA(launch_fused(en, p, 0, false));
-        constexpr int kReps = 3;
+        const int kReps = small ? 8 : 3;
         OEMS_CUDA(cudaEventRecord(en->ev0, en->stream));
         for (int r = 0; r < kReps; ++r) OEMS_CUDA(launch_fused(en, p, 0, false));
         OEMS_CUDA(cudaEventRecord(en->ev1, en->stream));

@@ -835,7 +835,11 @@ template <int kSteps, int kIdBytes, bool kCpml, typename T>
 __global__ void __launch_bounds__(kFusedMaxThreads, 1) k_fused(const __grid_constant__ FusedArgs a) {
   extern __shared__ __align__(16) char fused_mem[];
   const float *tab, *prof;
+  // the next pass may take this one's place on an SM as CTAs end; its own
+  // wait below keeps it from the fields until all of them have
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   fused_stage<kSteps, kIdBytes, kCpml, T>(a, fused_mem, tab, prof);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   int b = 0;
   while (b + 1 < a.nbox && (int)blockIdx.x >= a.box[b + 1].item0) ++b;
   const FusedBox& B = a.box[b];

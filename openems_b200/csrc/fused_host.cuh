@@ -518,6 +518,7 @@ static oems_status fused_tune(oems_engine* en) {
     for (bool cpml : {false, true})
       OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
+  if (en->cpml.on) side_stream(en);  // (not for the first time inside a capture)
   const bool time_it = !(en->flags & OEMS_ENGINE_NO_AUTOTUNE);
   const FusedKey key{en->device, en->nx, en->ny, en->nz, F.id_bytes, F.id_bytes == 1 ? F.ntable : 0,
                      fused_prof_floats(en), (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0)};
@@ -582,6 +583,7 @@ static oems_status fused_tune(oems_engine* en) {
 static oems_status fused_pack_tune(oems_engine* en, int sms) {
   FusedHost& F = en->fus;
   if (F.pack_sms == sms && F.tuned_pack) return OEMS_OK;
+  if (en->cpml.on) side_stream(en);  // (not for the first time inside a capture)
   int smem_cta = 0, smem_sm = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, en->device));

@@ -619,7 +619,8 @@ OEMS_API oems_status oems_engine_set_kernel_profiling(oems_engine* engine, int32
  * (2: staged on the box between the x / y CPML slabs, register kernels on
  * the slabs; 3: the z-split, plain register kernels on the CPML-free box and
  * CPML register kernels on every slab cell; 4: the pipelined register
- * kernels), threads per CTA, x-planes per work item, rows per tile (staged),
+ * kernels; 5: fused passes, whose steps per pass stand for the stages),
+ * threads per CTA, x-planes per work item, rows per tile (staged),
  * pipeline stages (staged, pipelined) or the L2 prefetch distance in
  * x-planes (register kernels, 0 = none), CTAs. */
 OEMS_API oems_status oems_engine_launch_info(const oems_engine* engine, int32_t* staged,
@@ -633,7 +634,9 @@ OEMS_API oems_status oems_engine_launch_info(const oems_engine* engine, int32_t*
  * registers with 512-thread CTAs, 1 / 2: 256-thread CTAs capped at 85 / 64
  * registers) + 1000 for a forked z-split slab launch (2000 with the interior
  * grid cut by one CTA per SM), the number of H + E pairs timed and their
- * device time in milliseconds. */
+ * device time in milliseconds.  Fused passes: threads + 1000 x those of the
+ * launch over the CPML slabs; extra = steps + 10 x chunks of a tile + 1000 x
+ * boxes; reps counts steps. */
 typedef struct oems_tune_entry {
   int32_t kind;
   int32_t threads;

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -579,10 +580,11 @@ struct FusedPlan {
   double cost = 0.0;
 };
 struct FusedKey {
-  int dev, nx, ny, nz, id_bytes, ntable, prof, mode;
+  int dev, nx, ny, nz, id_bytes, ntable, mode;
+  std::array<int, 6> layers;  // of the CPML: a plan's boxes follow its slabs
   bool operator<(const FusedKey& o) const {
-    return std::tie(dev, nx, ny, nz, id_bytes, ntable, prof, mode) <
-           std::tie(o.dev, o.nx, o.ny, o.nz, o.id_bytes, o.ntable, o.prof, o.mode);
+    return std::tie(dev, nx, ny, nz, id_bytes, ntable, mode, layers) <
+           std::tie(o.dev, o.nx, o.ny, o.nz, o.id_bytes, o.ntable, o.mode, o.layers);
   }
 };
 struct FusedHost {

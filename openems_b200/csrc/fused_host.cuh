@@ -500,8 +500,13 @@ static cudaError_t launch_fused(oems_engine* en, const FusedPlan& p, int local, 
   return cudaGetLastError();
 }
 
-static std::map<FusedKey, std::vector<FusedPlan>>& fused_cache() {
-  static std::map<FusedKey, std::vector<FusedPlan>> m;
+// Plans already tuned in this process, with the candidates that were timed.
+struct FusedTuned {
+  std::vector<FusedPlan> plans;
+  std::vector<oems_tune_entry> report;
+};
+static std::map<FusedKey, FusedTuned>& fused_cache() {
+  static std::map<FusedKey, FusedTuned> m;
   return m;
 }
 
@@ -520,14 +525,19 @@ static oems_status fused_tune(oems_engine* en) {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
   if (en->cpml.on) side_stream(en);  // (not for the first time inside a capture)
   const bool time_it = !(en->flags & OEMS_ENGINE_NO_AUTOTUNE);
+  std::array<int, 6> layers{};
+  if (en->cpml.on) std::copy(en->cpml.args.L, en->cpml.args.L + 6, layers.begin());
   const FusedKey key{en->device, en->nx, en->ny, en->nz, F.id_bytes, F.id_bytes == 1 ? F.ntable : 0,
-                     fused_prof_floats(en), (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0)};
+                     (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0), layers};
   std::vector<FusedPlan> plans;
   en->tune_report.clear();
   {
     std::lock_guard<std::mutex> lock(tune_mutex());
     auto hit = fused_cache().find(key);
-    if (hit != fused_cache().end()) plans = hit->second;
+    if (hit != fused_cache().end()) {
+      plans = hit->second.plans;
+      en->tune_report = hit->second.report;
+    }
   }
   const bool cached = !plans.empty();
   for (int steps = 1; steps <= 2; ++steps) {
@@ -571,7 +581,7 @@ static oems_status fused_tune(oems_engine* en) {
   }
   if (!cached) {
     std::lock_guard<std::mutex> lock(tune_mutex());
-    fused_cache()[key] = {F.plan[0], F.plan[1]};
+    fused_cache()[key] = FusedTuned{{F.plan[0], F.plan[1]}, en->tune_report};
   }
   F.tuned = true;
   en->graph_epoch++;

@@ -74,6 +74,15 @@ def test_sizes_against_separate_kernels(dims):
             same(run_engine(sc, compressed=True, graphs=False), ref)
 
 
+def test_one_grid_with_other_slabs():
+    """Engines of one size whose slabs lie on other faces each get boxes of
+    their own (plans are kept per grid and slab layout)."""
+    for layers in ((8, 0, 0, 0, 0, 0), (0, 8, 0, 0, 0, 0), (0, 0, 8, 0, 0, 0), (0, 0, 0, 8, 0, 0), (0, 0, 0, 0, 8, 0),
+                   (0, 0, 0, 0, 0, 8), (4, 4, 0, 0, 0, 0)):
+        sc = random_scenario(11, (70, 66, 130), layers)
+        same(run_engine(sc), run_engine(sc, kernels="register", autotune=False))
+
+
 @pytest.mark.parametrize("storage", ["f16", "bf16"])
 def test_two_byte_storage(storage):
     for layers in (None, (8, 0, 6, 10, 0, 9)):

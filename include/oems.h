@@ -372,7 +372,9 @@ OEMS_API oems_status oems_engine_reset(oems_engine* engine);
  * condition, and their engines must be at the same timestep; each engine
  * keeps its own decay threshold, peak and termination step.  statuses[i] is
  * OEMS_ERR_NUMERICAL for an engine whose energy stopped being finite (it
- * stops at that check), OEMS_OK otherwise.  The engines must not be used
+ * stops at that check), OEMS_OK otherwise.  An engine that has been given
+ * any other extension or a recorder since the pack was made is refused with
+ * OEMS_ERR_CONFIG before anything is launched.  The engines must not be used
  * elsewhere while a pack call runs; destroy the pack before its engines. */
 typedef struct oems_pack oems_pack;
 OEMS_API oems_status oems_pack_create(oems_engine* const* engines, uint64_t count, oems_pack** out);

@@ -4437,6 +4437,13 @@ static oems_status pack_fused(oems_pack* p, const std::vector<int>& part, bool* 
   return OEMS_OK;
 }
 
+// What a pack steps: extensions and recorders have no part in its launches (a
+// recorder's tables are filled by run_batch only).
+static bool pack_takes(const oems_engine* en) {
+  return !(en->mur.on || en->upml.on || en->tfsf.on || !en->disp.empty() || !en->rlc.q.empty() || !en->fdumps.empty() ||
+           !en->boxes.empty());
+}
+
 static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches, oems_batch_result* results,
                                   oems_status* statuses) {
   const auto t_start = std::chrono::steady_clock::now();
@@ -4453,6 +4460,10 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
         b->check_interval != b0->check_interval || b->has_energy_decay_db != b0->has_energy_decay_db ||
         p->en[i]->timestep != p->en[part.empty() ? i : part[0]]->timestep)
       return fail(OEMS_ERR_CONFIG, "the batches of a pack must share step count, intervals and start step");
+    // (one may have been added since the pack was made)
+    if (!pack_takes(p->en[i]))
+      return fail(OEMS_ERR_CONFIG, "engine " + std::to_string(i) +
+                                       ": a pack runs CPML, sources, probes and probe DFTs only");
     part.push_back((int)i);
   }
   if (part.empty()) return OEMS_OK;
@@ -4640,9 +4651,7 @@ oems_status oems_pack_create(oems_engine* const* engines, uint64_t count, oems_p
     if (en->device != engines[0]->device) return fail(OEMS_ERR_CONFIG, "the engines of a pack share one device");
     if (en->storage != engines[0]->storage) return fail(OEMS_ERR_CONFIG, "the engines of a pack share one field storage");
     if (en->id_bytes != 0) return fail(OEMS_ERR_CONFIG, "a pack needs full coefficient arrays");
-    if (en->mur.on || en->upml.on || en->tfsf.on || !en->disp.empty() || !en->rlc.q.empty() || !en->fdumps.empty() ||
-        !en->boxes.empty())
-      return fail(OEMS_ERR_CONFIG, "a pack runs CPML, sources, probes and probe DFTs only");
+    if (!pack_takes(en)) return fail(OEMS_ERR_CONFIG, "a pack runs CPML, sources, probes and probe DFTs only");
     for (uint64_t j = 0; j < i; ++j)
       if (engines[j] == en) return fail(OEMS_ERR_CONFIG, "an engine appears twice in the pack");
   }

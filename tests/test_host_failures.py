@@ -1,0 +1,97 @@
+"""What the engine library's host code does when a call fails or a limit is
+reached: the library's own sources built against fake_cudart.cpp (device
+memory on the host, kernels that only leave their names), each test in a
+process of its own."""
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from openems_b200 import build as engine_build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+OUT = os.path.join(HERE, "_build")
+LIB = os.path.join(OUT, "liboems_fake.so")
+
+HEAD = """
+import ctypes, sys
+import numpy as np
+import openems_b200._native as N
+N.LIB_PATH = %r
+import openems_b200 as oe
+L, F = N.lib(), ctypes.CDLL(N.LIB_PATH)
+for f in ("fake_launched", "fake_pool_used", "fake_pinned", "fake_instantiated"):
+    getattr(F, f).restype = ctypes.c_longlong
+F.fake_set.argtypes = [ctypes.c_char_p, ctypes.c_longlong]
+
+def knob(key, value):
+    F.fake_set(key.encode(), value)
+
+def launched(part, reset=False):
+    return F.fake_launched(part.encode(), int(reset))
+
+def engine(dims, layers=None, **kw):
+    e = oe.Engine(oe.Operator(oe.Grid.uniform(*dims, 1e-3), oe.BoundaryConditions.all_pec()), **kw)
+    if layers:
+        e.add_cpml(oe.CpmlBoundaries(layers=layers))
+    return e
+
+def batch(n):
+    return oe.EngineBatch(num_steps=n)
+
+def fused(e):
+    return e.launch_info()["staged"] == 5
+"""
+
+
+@pytest.fixture(scope="module")
+def child():
+    os.makedirs(OUT, exist_ok=True)
+    csrc = os.path.join(engine_build.HERE, "csrc")
+    fake = os.path.join(HERE, "fake_cudart.cpp")
+    deps = [fake] + [os.path.join(csrc, f) for f in os.listdir(csrc)] + \
+           [os.path.join(engine_build.ROOT, "include", f) for f in os.listdir(os.path.join(engine_build.ROOT, "include"))]
+    if not os.path.exists(LIB) or max(map(os.path.getmtime, deps)) > os.path.getmtime(LIB):
+        flags = ["-gencode", "arch=compute_100a,code=compute_100a", "-O1", "-Xcicc", "-O0", "-std=c++17", "-Xcompiler",
+                 "-fPIC", "--expt-relaxed-constexpr", "-I", os.path.join(engine_build.ROOT, "include")]
+        jobs, objs = [], []
+        for src in [os.path.join(engine_build.HERE, s) for s in engine_build.SOURCES] + [fake]:
+            objs.append(os.path.join(OUT, os.path.basename(src) + ".o"))
+            jobs.append(subprocess.Popen([engine_build._nvcc(), *flags, "-c", src, "-o", objs[-1]]))
+        assert [j.wait() for j in jobs] == [0] * len(jobs)
+        subprocess.run(["g++", "-shared", "-Wl,--no-undefined", "-o", LIB + ".tmp", *objs, "-lpthread", "-ldl"], check=True)
+        os.replace(LIB + ".tmp", LIB)
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", HEAD % LIB + textwrap.dedent(code)], cwd=engine_build.ROOT,
+                           capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-3000:]
+    return run
+
+
+@pytest.mark.parametrize("add", [
+    "oe.fdtd.Nf2ffBox(e[1], (4, 4, 4), (15, 15, 15), [1e9])",
+    "e[1].add_mur(oe.MurAbcConfig.all(1))",
+    "e[1].add_dispersive(oe.DrudeMaterial(2e11, 1e9), np.array([[8, 8, 8]], dtype=np.uint64))",
+])
+def test_pack_refuses_what_was_added_after_it_was_made(child, add):
+    """A recorder's tables are filled for its own engine's batches only: the
+    pack's passes would read none, or another batch's."""
+    child(f"""
+    e = [engine((20, 20, 20)) for _ in range(2)]
+    p = oe.Pack(e)
+    p.run_batch([batch(4), batch(4)])
+    {add}
+    launched("", True)
+    try:
+        p.run_batch([batch(4), batch(4)])
+    except oe.ConfigError:
+        pass
+    else:
+        raise AssertionError("accepted")
+    assert launched("") == 0
+    p.run_batch([batch(4), None])  # the others go on
+    assert launched("k_fused") > 0
+    """)

@@ -2114,14 +2114,11 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
   en->last_launches = 0;
   bool fused = false;
   OEMS_TRY(fused_ready(en, &fused));
+  if (fused && !en->fus.tuned) OEMS_TRY(fused_tune(en, &fused));
   if (fused != en->fus.use || en->fus.packed) en->graph_epoch++;
   en->fus.use = fused;
   en->fus.packed = false;
-  if (fused) {
-    if (!en->fus.tuned) OEMS_TRY(fused_tune(en));
-  } else if (!en->tuned) {
-    OEMS_TRY(autotune(en));
-  }
+  if (!fused && !en->tuned) OEMS_TRY(autotune(en));
   const int prev_nexc = en->nexc;
   OEMS_TRY(upload_excitations(en, b));
   if (prev_nexc != en->nexc) en->graph_epoch++;  // nexc is baked into captured graphs
@@ -4429,7 +4426,12 @@ static oems_status pack_fused(oems_pack* p, const std::vector<int>& part, bool* 
     // shapes for the engine's share of the device: with the others filling
     // the rest, long x-runs and full tiles beat many short items
     const int share = std::max(1, std::min(sms, (int)std::lround(sms * (double)en->ncells_padded / cells)));
-    OEMS_TRY(fused_pack_tune(en, share));
+    bool ok = false;
+    OEMS_TRY(fused_pack_tune(en, share, &ok));
+    if (!ok) return OEMS_OK;
+  }
+  for (int i : part) {
+    oems_engine* en = p->en[i];
     if (!en->fus.use || !en->fus.packed) en->graph_epoch++;
     en->fus.use = en->fus.packed = true;
   }

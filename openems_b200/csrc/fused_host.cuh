@@ -308,13 +308,23 @@ static double fused_item_cost(const FusedPlan& p, int b, int planes, const int (
   return (planes + (p.steps == 2 ? 4.5 : 2.5)) * std::max(latency, slots) / occ[c];
 }
 
+// Most items an SM of plans that cut x into runs: past that, shorter runs only
+// add lead-in planes.  (A plan of one run is always a candidate: its items
+// follow the size of the (y, z) plane, whatever the number of SMs.)
+constexpr int kFusedItems = 16;
+
 static double fused_cost(const FusedPlan& p, int sms, const int (&occ)[2], std::vector<double>& heap) {
   heap.assign(sms, 0.0);
   for (int b = 0; b < p.nbox; ++b) {
     const FusedBox& B = p.box[b];
     for (int i = B.i0; i < B.i1; i += B.xlen) {
       const double t = fused_item_cost(p, b, std::min(B.xlen, B.i1 - i), occ);
-      for (int k = 0; k < B.ntz * B.nty; ++k) {
+      int left = B.ntz * B.nty;
+      if (left > kFusedItems * sms) {  // a very wide plane: whole rounds of the SMs at once
+        for (double& h : heap) h += (left / sms) * t;
+        left %= sms;
+      }
+      for (int k = 0; k < left; ++k) {
         std::pop_heap(heap.begin(), heap.end(), std::greater<double>());
         heap.back() += t;
         std::push_heap(heap.begin(), heap.end(), std::greater<double>());
@@ -396,7 +406,7 @@ static std::vector<FusedPlan> fused_shapes(const oems_engine* en, int steps, int
         B.item0 = p.items[k];
         p.items[k] += B.ntz * B.nty * ((all_b + B.xlen - 1) / B.xlen);
       }
-      if (p.items[0] + p.items[1] > 16 * sms) break;
+      if (n > 1 && p.items[0] + p.items[1] > kFusedItems * sms) break;
       p.cost = fused_cost(p, sms, occ, heap);
       kept.push_back(p);
     }
@@ -512,9 +522,12 @@ static std::map<FusedKey, FusedTuned>& fused_cache() {
 
 // Tile shapes of the one- and two-step passes: the model's best, or (with
 // the autotuner) the fastest of its first few on the engine's own state,
-// which a pass only reads.
-static oems_status fused_tune(oems_engine* en) {
+// which a pass only reads.  *ok: false where a CTA's shared memory takes no
+// tile at all (CPML profiles of thousands of layers): the engine then keeps
+// the separate kernels.
+static oems_status fused_tune(oems_engine* en, bool* ok) {
   FusedHost& F = en->fus;
+  *ok = false;
   int sms = 0, smem_cta = 0, smem_sm = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, en->device));
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
@@ -542,14 +555,19 @@ static oems_status fused_tune(oems_engine* en) {
   const bool cached = !plans.empty();
   for (int steps = 1; steps <= 2; ++steps) {
     std::vector<FusedPlan> c;
-    if (cached)
+    const bool have = cached && plans[steps - 1].nbox > 0;
+    if (have)
       c.push_back(plans[steps - 1]);
     else
       c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
-    if (c.empty()) return fail(OEMS_ERR_CUDA, "no tile shape of the fused kernels fits this device");
+    if (c.empty()) {
+      if (steps > fused_max_steps(en)) continue;
+      F.state = -1;
+      return OEMS_OK;
+    }
     // one-step passes only finish odd spans unless an extension needs them
     const bool small = en->ncells_padded < kFusedSmall;
-    const size_t most = cached || !time_it ? 1 : steps != fused_max_steps(en) ? 3 : small ? 30 : 12;
+    const size_t most = have || !time_it ? 1 : steps != fused_max_steps(en) ? 3 : small ? 30 : 12;
     if (c.size() > most) c.resize(most);
     FusedPlan best = c[0];
     if (c.size() > 1) {
@@ -583,16 +601,21 @@ static oems_status fused_tune(oems_engine* en) {
     std::lock_guard<std::mutex> lock(tune_mutex());
     fused_cache()[key] = FusedTuned{{F.plan[0], F.plan[1]}, en->tune_report};
   }
-  F.tuned = true;
+  F.tuned = *ok = true;
   en->graph_epoch++;
   return OEMS_OK;
 }
 
 // Shapes for an engine that shares the device with others: the model's best
-// on `sms` SMs.
-static oems_status fused_pack_tune(oems_engine* en, int sms) {
+// on `sms` SMs.  *ok as for fused_tune.
+static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
   FusedHost& F = en->fus;
-  if (F.pack_sms == sms && F.tuned_pack) return OEMS_OK;
+  const int most = fused_max_steps(en);
+  if (F.pack_sms == sms && F.tuned_pack) {
+    *ok = F.pack_plan[most - 1].nbox > 0;
+    return OEMS_OK;
+  }
+  F.pack_plan[0] = F.pack_plan[1] = FusedPlan{};
   if (en->cpml.on) side_stream(en);  // (not for the first time inside a capture)
   int smem_cta = 0, smem_sm = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
@@ -602,9 +625,10 @@ static oems_status fused_pack_tune(oems_engine* en, int sms) {
       OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
     const std::vector<FusedPlan> c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
-    if (c.empty()) return fail(OEMS_ERR_CUDA, "no tile shape of the fused kernels fits this device");
+    if (c.empty()) break;
     F.pack_plan[steps - 1] = c[0];
   }
+  *ok = F.pack_plan[most - 1].nbox > 0;
   F.pack_sms = sms;
   F.tuned_pack = true;
   en->graph_epoch++;

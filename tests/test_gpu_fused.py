@@ -74,6 +74,14 @@ def test_sizes_against_separate_kernels(dims):
             same(run_engine(sc, compressed=True, graphs=False), ref)
 
 
+@pytest.mark.parametrize("dims,layers", [((2, 2300, 2310), None), ((8, 2000, 2000), (2, 2, 8, 8, 8, 8))])
+def test_wide_planes(dims, layers):
+    """More tiles in one (y, z) plane than 16 items an SM."""
+    sc = random_scenario(12, dims, layers, steps=17)
+    sc.batches = (12, 5)
+    same(run_engine(sc, autotune=False), run_engine(sc, kernels="register", autotune=False))
+
+
 def test_one_grid_with_other_slabs():
     """Engines of one size whose slabs lie on other faces each get boxes of
     their own (plans are kept per grid and slab layout)."""

@@ -6,7 +6,7 @@ import pytest
 
 import openems_b200 as oe
 from openems_b200.sweep import Sweep
-from scenarios import cpml_scenarios, make_operator, odd_scenarios, reference_scenarios
+from scenarios import Scenario, cpml_scenarios, make_operator, odd_scenarios, reference_scenarios
 from test_gpu_sweep import FREQS, instances
 
 pytestmark = pytest.mark.gpu
@@ -176,3 +176,24 @@ def test_packed_sweep_equals_sweep(cap):
             r, f = sw.result(iid), ref.result(rid)
             assert r["timesteps"] == f["timesteps"] and not r["paused"]
             assert np.array_equal(r["uf"], f["uf"]) and np.array_equal(r["if"], f["if"])
+
+
+def test_small_shares_of_the_device():
+    """An engine whose share of the SMs is one or two, with a wide (y, z) plane."""
+    def scenes():
+        out = []
+        for dims, layers in (((4, 300, 300), None), ((10, 320, 290), (2, 2, 8, 8, 8, 8)), ((150, 200, 210), (8,) * 6)):
+            sc = Scenario(f"share_{dims[0]}", dims, 1e-3, excitations=[
+                oe.Excitation.gaussian_pulse(2e-11, 1e-11, 2, tuple(d // 2 for d in dims))], num_steps=40,
+                probes=[(2, tuple(d // 2 + 1 for d in dims))])
+            sc.cpml = oe.CpmlBoundaries(layers=layers) if layers else None
+            out.append(sc)
+        return out
+    alone, packed = [_engine(sc) for sc in scenes()], [_engine(sc) for sc in scenes()]
+    pack = oe.Pack([e for _, e in packed])
+    pack.run_batch([_batch(sc, op, 0, 40) for sc, (op, _) in zip(scenes(), packed)])
+    for sc, (op, a), (_, b) in zip(scenes(), alone, packed):
+        a.run_batch(_batch(sc, op, 0, 40))
+        assert b.launch_info()["staged"] == 5
+        assert np.array_equal(np.stack(a.read_fields()), np.stack(b.read_fields()))
+        assert np.array_equal(a.probe_traces(), b.probe_traces())

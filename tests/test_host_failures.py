@@ -95,3 +95,37 @@ def test_pack_refuses_what_was_added_after_it_was_made(child, add):
     p.run_batch([batch(4), None])  # the others go on
     assert launched("k_fused") > 0
     """)
+
+
+# 64 items of 2,048 cells fill four SMs' limit of 16 items each; a whole
+# (y, z) plane of these grids takes more
+@pytest.mark.parametrize("dims,layers", [((8, 500, 500), None), ((1, 600, 600), None), ((24, 400, 400), (8,) * 6)])
+@pytest.mark.parametrize("autotune", [True, False])
+def test_wide_planes_have_a_plan(child, dims, layers, autotune):
+    child(f"""
+    knob("sms", 4)
+    e = engine({dims}, {layers}, autotune={autotune})
+    e.run_batch(batch(5))
+    assert fused(e) and launched("k_fused") > 0
+    """)
+
+
+def test_pack_of_small_shares_has_plans(child):
+    """An engine beside much larger ones plans for one SM."""
+    child("""
+    e = [engine((1, 300, 300)), engine((4, 300, 300), (1, 1, 8, 8, 8, 8)), engine((40, 300, 300))]
+    knob("sms", 8)
+    oe.Pack(e).run_batch([batch(5)] * 3)
+    assert all(map(fused, e)) and launched("k_update") == 0
+    """)
+
+
+def test_profiles_beyond_shared_memory_keep_the_separate_kernels(child):
+    """6 x 4 B x 20,000 layers of one profile: no CTA holds them."""
+    child("""
+    e = [engine((20010, 3, 3), (20000, 0, 0, 0, 0, 0)) for _ in range(2)]
+    e[0].run_batch(batch(5))
+    assert not fused(e[0]) and launched("k_update_h") > 0 and launched("k_fused") == 0
+    oe.Pack(e[1:]).run_batch([batch(5)])
+    assert launched("k_update_h_pack") > 0 and launched("k_fused") == 0
+    """)

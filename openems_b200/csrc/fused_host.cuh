@@ -34,9 +34,28 @@ static int fused_max_steps(const oems_engine* en) {
   return fused_hooks(en) || !en->fdumps.empty() || !en->boxes.empty() || qa > qb ? 1 : 2;
 }
 
+// Whether there is room; a refusal is not an error of the batch, the engine
+// goes on without what the buffer was for.
+template <typename... A>
+static bool got_room(A... allocated) {
+  const bool ok = ((allocated == cudaSuccess) && ...);
+  if (!ok) cudaGetLastError();
+  return ok;
+}
+
+// Gives back what fused passes hold beside the engine's own buffers.
+static void fused_release(oems_engine* en) {
+  FusedHost& F = en->fus;
+  F.own_ids.release();
+  F.own_table.release();
+  F.alt.release();
+  F.psi.release();
+}
+
 // Ids and table of the distinct coefficient sets of a full-array engine, by
-// two kernels over the arrays.  More than 65,536 sets, or two sets with one
-// hash: the engine keeps its full arrays and the register kernels.
+// two kernels over the arrays.  More than 65,536 sets, two sets with one hash
+// or no room for the tables: the engine keeps its full arrays and the
+// register kernels.
 static oems_status fused_ids(oems_engine* en, bool* ok) {
   FusedHost& F = en->fus;
   *ok = false;
@@ -51,11 +70,9 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   DevBuf<unsigned long long> key;
   DevBuf<long long> rep;
   DevBuf<int> list, count, id_of;
-  OEMS_CUDA(key.ensure(kCoefSlots));
-  OEMS_CUDA(rep.ensure(kCoefSlots));
-  OEMS_CUDA(list.ensure(kCoefMax));
-  OEMS_CUDA(count.ensure(2));
-  OEMS_CUDA(id_of.ensure(kCoefSlots));
+  if (!got_room(key.ensure(kCoefSlots), rep.ensure(kCoefSlots), list.ensure(kCoefMax), count.ensure(2),
+                id_of.ensure(kCoefSlots)))
+    return OEMS_OK;
   OEMS_CUDA(cudaMemsetAsync(key.p, 0, kCoefSlots * sizeof(*key.p), en->stream));
   OEMS_CUDA(cudaMemsetAsync(rep.p, 0x7f, kCoefSlots * sizeof(*rep.p), en->stream));
   OEMS_CUDA(cudaMemsetAsync(count.p, 0, 2 * sizeof(int), en->stream));
@@ -78,7 +95,7 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   OEMS_CUDA(cudaStreamSynchronize(en->stream));
   if (n[1] || n[0] > kCoefMax) return OEMS_OK;
   DevBuf<long long> first;
-  OEMS_CUDA(first.ensure(n[0]));
+  if (!got_room(first.ensure(n[0]))) return OEMS_OK;
   k_coef_first<<<blocks_for(n[0], 256), 256, 0, en->stream>>>(list.p, rep.p, n[0], first.p);
   OEMS_CUDA(cudaGetLastError());
   std::vector<std::pair<long long, int>> sets(n[0]);
@@ -96,8 +113,8 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   }
   F.id_bytes = n[0] <= 256 ? 1 : 2;
   F.ntable = n[0];
-  OEMS_CUDA(F.own_ids.ensure((size_t)en->ncells_padded * F.id_bytes));
-  OEMS_CUDA(F.own_table.ensure((size_t)n[0] * 12));
+  if (!got_room(F.own_ids.ensure((size_t)en->ncells_padded * F.id_bytes), F.own_table.ensure((size_t)n[0] * 12)))
+    return OEMS_OK;
   OEMS_CUDA(cudaMemsetAsync(F.own_ids.p, 0, (size_t)en->ncells_padded * F.id_bytes, en->stream));
   OEMS_CUDA(cudaMemcpyAsync(list.p, slots.data(), n[0] * sizeof(int), cudaMemcpyHostToDevice, en->stream));
   OEMS_CUDA(cudaMemcpyAsync(first.p, cells.data(), n[0] * sizeof(long long), cudaMemcpyHostToDevice, en->stream));
@@ -112,11 +129,7 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   OEMS_CUDA(cudaGetLastError());
   OEMS_CUDA(cudaMemcpyAsync(n, count.p, sizeof(n), cudaMemcpyDeviceToHost, en->stream));
   OEMS_CUDA(cudaStreamSynchronize(en->stream));
-  if (n[1]) {
-    F.own_ids.release();
-    F.own_table.release();
-    return OEMS_OK;
-  }
+  if (n[1]) return OEMS_OK;
   F.ids = F.own_ids.p;
   F.table = F.own_table.p;
   *ok = true;
@@ -143,9 +156,8 @@ static oems_status fused_ready(oems_engine* en, bool* yes) {
     if (need > free_b / 4) return OEMS_OK;
     bool ok = false;
     OEMS_TRY(fused_ids(en, &ok));
-    if (!ok) return OEMS_OK;
-    if (F.alt.ensure(en->field_bytes()) != cudaSuccess) {
-      cudaGetLastError();
+    if (!ok || !got_room(F.alt.ensure(en->field_bytes()))) {
+      fused_release(en);
       return OEMS_OK;
     }
     // pads and rows no pass writes stay 0, as in the first buffers
@@ -153,9 +165,9 @@ static oems_status fused_ready(oems_engine* en, bool* yes) {
     F.state = 1;
   }
   if (en->cpml.on && F.psi.n != en->cpml.psi.n) {
-    if (F.psi.ensure(en->cpml.psi.n) != cudaSuccess) {
-      cudaGetLastError();
+    if (!got_room(F.psi.ensure(en->cpml.psi.n))) {
       F.state = -1;
+      fused_release(en);
       return OEMS_OK;
     }
     OEMS_CUDA(cudaMemsetAsync(F.psi.p, 0, F.psi.n * sizeof(float), en->stream));
@@ -563,6 +575,7 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
     if (c.empty()) {
       if (steps > fused_max_steps(en)) continue;
       F.state = -1;
+      fused_release(en);
       return OEMS_OK;
     }
     // one-step passes only finish odd spans unless an extension needs them
@@ -636,7 +649,7 @@ static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
 }
 
 // Longest spans of a batch, and the tap buffers for them.
-static oems_status fused_taps_ready(oems_engine* en, uint64_t span);
+static oems_status fused_taps_ready(oems_engine* en, uint64_t span, bool* room);
 static uint64_t fused_span_cap(const oems_engine* en);
 static oems_status fused_spans(oems_engine* en, const oems_batch* b, uint64_t* cap) {
   if (en->nprobe() == 0) return OEMS_OK;
@@ -645,7 +658,15 @@ static oems_status fused_spans(oems_engine* en, const oems_batch* b, uint64_t* c
   if (b->sample_interval > 0) longest = std::min<uint64_t>(longest, b->sample_interval);
   // (the first check comes after step check_interval, not after step 0)
   if (b->has_energy_decay_db && b->check_interval > 0) longest = std::min<uint64_t>(longest, b->check_interval + 1);
-  return fused_taps_ready(en, longest);
+  // shorter spans where there is no room for the longest one's taps
+  for (;; longest /= 2) {
+    bool room = false;
+    OEMS_TRY(fused_taps_ready(en, longest, &room));
+    if (room) break;
+    if (longest <= 1) return fail(OEMS_ERR_CUDA, "no device memory for the probes' values of one step");
+    *cap = longest / 2;
+  }
+  return OEMS_OK;
 }
 
 // Sources of the batch sorted by (plane, row, chunk); equal cells keep the
@@ -694,9 +715,10 @@ static uint64_t fused_span_cap(const oems_engine* en) {
 }
 
 // Tap tables (after probes were added) and the buffer of a batch's longest span.
-static oems_status fused_taps_ready(oems_engine* en, uint64_t span) {
+static oems_status fused_taps_ready(oems_engine* en, uint64_t span, bool* room) {
   FusedHost& F = en->fus;
   const int n = (int)en->term_idx.size();
+  *room = true;
   if (n == 0) return OEMS_OK;
   if (F.ntap != n) {
     const int nzp = en->g.nzp, nzq = en->g.nzq;
@@ -730,7 +752,7 @@ static oems_status fused_taps_ready(oems_engine* en, uint64_t span) {
   }
   const size_t need = (size_t)std::max<uint64_t>(span, 1) * n;
   if (F.taps.n < need) {
-    OEMS_CUDA(F.taps.ensure(need));
+    *room = got_room(F.taps.ensure(need));
     en->graph_epoch++;
   }
   return OEMS_OK;

@@ -129,3 +129,26 @@ def test_profiles_beyond_shared_memory_keep_the_separate_kernels(child):
     oe.Pack(e[1:]).run_batch([batch(5)])
     assert launched("k_update_h_pack") > 0 and launched("k_fused") == 0
     """)
+
+
+# the sets' hash table is 2 MB; ids 1.1 MB; the second fields 26 MB; psi 5 MB
+@pytest.mark.parametrize("refused", [2 << 20, 1 << 20, 20 << 20, 4 << 20])
+def test_no_room_for_fused_buffers_keeps_the_separate_kernels(child, refused):
+    child(f"""
+    e = engine((100, 100, 110), (8,) * 6, autotune=False)
+    used = F.fake_pool_used()
+    knob("fail_pool_from", {refused})
+    e.run_batch(batch(5))
+    assert not fused(e) and launched("k_update_h") > 0
+    assert F.fake_pool_used() - used < 1 << 20  # nothing of the attempt stays
+    """)
+
+
+def test_no_room_for_taps_shortens_the_spans(child):
+    child("""
+    e = engine((30, 150, 150))
+    e.add_probe(oe.fdtd.current_probe((15, 20, 20), (15, 120, 120), 0))
+    e.run_batch(batch(2))
+    knob("fail_pool_from", 1 << 20)
+    assert e.run_batch(batch(3000)).timesteps_executed == 3000 and fused(e)
+    """)

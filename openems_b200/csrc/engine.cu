@@ -1498,8 +1498,14 @@ static std::mutex& tune_mutex();
 static oems_status launch_steps_fused(oems_engine* en, int steps);
 static uint64_t fused_launches(const oems_engine* en, int steps);
 static void fused_swap(oems_engine* en);
+static void fused_rewind(oems_engine* en, int parity) {
+  if (en->fus.parity != parity) fused_swap(en);
+}
 static int fused_max_steps(const oems_engine* en);
 
+// The graph of `steps` steps from the current buffers.  On success the current
+// buffers are the ones it will have written last; a caller whose launch fails
+// goes back to those before, as a failure here does.
 static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
   if (en->built_epoch != en->graph_epoch) {
     drop_graphs(en);
@@ -1517,18 +1523,20 @@ static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
   }
   if (en->graphs.size() >= 8) drop_graphs(en);
   cudaGraph_t graph = nullptr;
+  const int parity = en->fus.parity;
   OEMS_CUDA(cudaStreamBeginCapture(en->stream, cudaStreamCaptureModeThreadLocal));
   oems_status st = en->fus.use ? launch_steps_fused(en, steps) : launch_steps_direct(en, steps);
   cudaError_t ce = cudaStreamEndCapture(en->stream, &graph);
+  cudaGraphExec_t exec = nullptr;
+  if (st == OEMS_OK && ce != cudaSuccess)
+    st = fail(OEMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
+  if (st == OEMS_OK && (ce = cudaGraphInstantiate(&exec, graph, 0)) != cudaSuccess)
+    st = fail(OEMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
+  if (graph) cudaGraphDestroy(graph);
   if (st != OEMS_OK) {
-    if (graph) cudaGraphDestroy(graph);
+    fused_rewind(en, parity);
     return st;
   }
-  if (ce != cudaSuccess) return fail(OEMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
-  cudaGraphExec_t exec = nullptr;
-  ce = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (ce != cudaSuccess) return fail(OEMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
   en->graphs[key] = exec;
   *out = exec;
   return OEMS_OK;
@@ -1553,8 +1561,11 @@ static oems_status run_span(oems_engine* en, long long base, int steps) {
     OEMS_TRY(launch_steps_direct(en, steps));
   } else {
     cudaGraphExec_t exec = nullptr;
+    const int parity = en->fus.parity;
     OEMS_TRY(get_graph(en, steps, &exec));
-    OEMS_CUDA(cudaGraphLaunch(exec, en->stream));
+    const cudaError_t e = cudaGraphLaunch(exec, en->stream);
+    if (e != cudaSuccess) fused_rewind(en, parity);
+    OEMS_CUDA(e);
   }
   en->last_launches += en->fus.use ? fused_launches(en, steps) : (uint64_t)steps * kernels_per_step(en);
   return OEMS_OK;

@@ -152,3 +152,34 @@ def test_no_room_for_taps_shortens_the_spans(child):
     knob("fail_pool_from", 1 << 20)
     assert e.run_batch(batch(3000)).timesteps_executed == 3000 and fused(e)
     """)
+
+
+# of the three kernel launches (two passes of 3 steps, the first swaps the
+# buffers), the second fails; the graph cannot be made; it cannot be launched
+@pytest.mark.parametrize("knobs", ['knob("pass_kernel", 1), knob("fail_kernel", 1)', 'knob("fail_instantiate", 1)',
+                                   'knob("fail_graph_launch", 1)'])
+@pytest.mark.parametrize("layers,again", [(None, False), ((4,) * 6, True)])
+def test_a_graph_that_fails_leaves_the_fields_current(child, knobs, layers, again):
+    """(Kernels do nothing here: what was written must come back.)"""
+    child(f"""
+    e = engine((20, 21, 22), {layers}, autotune=False)
+    e.run_batch(batch(2))  # (tables and buffers are there)
+    steps = 1 if "kernel" not in {knobs!r} else 3
+    if {again}:  # a graph kept from before, launched again
+        for _ in range(2):
+            e.run_batch(batch(steps))
+            e.run_batch(batch(steps + 4))
+        steps = steps if "launch" in {knobs!r} else steps + 8
+    f = np.random.default_rng(0).standard_normal((2, 3, 20, 21, 22), dtype=np.float32)
+    e.write_fields(f[0], f[1])
+    {knobs}
+    try:
+        e.run_batch(batch(steps))
+    except N.CudaError:
+        pass
+    else:
+        raise AssertionError("no error")
+    assert fused(e)
+    got = e.read_fields()
+    assert np.array_equal(got[0], f[0]) and np.array_equal(got[1], f[1])
+    """)

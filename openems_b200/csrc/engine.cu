@@ -1503,6 +1503,9 @@ static void fused_rewind(oems_engine* en, int parity) {
 }
 static int fused_max_steps(const oems_engine* en);
 
+// Span lengths whose graphs are kept (each may need one per buffer parity).
+constexpr size_t kMaxGraphs = 16;
+
 // The graph of `steps` steps from the current buffers.  On success the current
 // buffers are the ones it will have written last; a caller whose launch fails
 // goes back to those before, as a failure here does.
@@ -1521,7 +1524,7 @@ static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
     }
     return OEMS_OK;
   }
-  if (en->graphs.size() >= 8) drop_graphs(en);
+  if (en->graphs.size() >= kMaxGraphs) drop_graphs(en);
   cudaGraph_t graph = nullptr;
   const int parity = en->fus.parity;
   OEMS_CUDA(cudaStreamBeginCapture(en->stream, cudaStreamCaptureModeThreadLocal));

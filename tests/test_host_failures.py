@@ -183,3 +183,19 @@ def test_a_graph_that_fails_leaves_the_fields_current(child, knobs, layers, agai
     got = e.read_fields()
     assert np.array_equal(got[0], f[0]) and np.array_equal(got[1], f[1])
     """)
+
+
+def test_graphs_of_both_parities_are_kept(child):
+    """Eight span lengths were kept before a span had a graph per parity."""
+    child("""
+    e = engine((20, 21, 22), autotune=False)
+    lengths = (1, 3, 5, 9, 11, 13, 17, 19)
+    for _ in range(2):
+        for n in lengths:
+            e.run_batch(batch(n))
+    before = F.fake_instantiated()
+    for _ in range(3):
+        for n in lengths:
+            e.run_batch(batch(n))
+    assert F.fake_instantiated() == before
+    """)

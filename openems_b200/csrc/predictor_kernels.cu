@@ -56,12 +56,18 @@ oems_status err_word(int** out) {
   return OEMS_OK;
 }
 
-// Stream-ordered workspace of one call.
+// Stream-ordered workspace of one call.  get: false where it is not to be
+// had, and the call takes the form that needs none.
 struct Workspace {
   void* p = nullptr;
   cudaStream_t s;
   explicit Workspace(void* stream) : s(reinterpret_cast<cudaStream_t>(stream)) {}
-  cudaError_t get(size_t bytes) { return oems::pool_alloc(&p, bytes, s); }
+  bool get(size_t bytes) {
+    if (oems::pool_alloc(&p, bytes, s) == cudaSuccess) return true;
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
   ~Workspace() {
     if (p) cudaFreeAsync(p, s);
   }
@@ -472,28 +478,28 @@ oems_status oems_tc_gemm_bf16(const void* a, int lda, const void* b, int ldb, fl
   // 65,536 ran on 10 of 148 SMs, 215 us): the K range in parts of at least 8
   // blocks, as many as the SMs take in one wave.  Fewer than half the SMs
   // busy, or the sum of the parts costs more than it gives.
+  const int nkb = (K + 63) / 64;
   p.splits = 1;
-  p.kb_per = (K + 63) / 64;
-  if (tm * ((N + BN - 1) / BN) * 2 <= sms && p.kb_per >= 32) {
+  p.kb_per = nkb;
+  Workspace ws(stream);
+  if (tm * ((N + BN - 1) / BN) * 2 <= sms && nkb >= 32) {
     long long fewest = -1;
     int split_bn = BN;
     for (int cand : {256, 128, 64}) {
       const long long t = tm * ((N + cand - 1) / cand);
-      const long long parts = std::max<long long>(1, std::min<long long>(sms / t, p.kb_per / 8));
-      const long long cost = ((p.kb_per + parts - 1) / parts) * (cand + 64);
+      const long long parts = std::max<long long>(1, std::min<long long>(sms / t, nkb / 8));
+      const long long cost = ((nkb + parts - 1) / parts) * (cand + 64);
       if (t <= sms && (fewest < 0 || cost < fewest)) fewest = cost, split_bn = cand;
     }
-    BN = split_bn;
-    const long long t = tm * ((N + BN - 1) / BN);
-    const int nkb = p.kb_per;
+    const long long t = tm * ((N + split_bn - 1) / split_bn);
     const int parts = (int)std::max<long long>(1, std::min<long long>(sms / t, nkb / 8));
-    p.kb_per = (nkb + parts - 1) / parts;
-    p.splits = (nkb + p.kb_per - 1) / p.kb_per;
-  }
-  Workspace ws(stream);
-  if (p.splits > 1) {
-    PK_CUDA(ws.get((size_t)p.splits * M * N * sizeof(float)));
-    p.part = static_cast<float*>(ws.p);
+    const int per = (nkb + parts - 1) / parts, splits = (nkb + per - 1) / per;
+    if (splits == 1 || ws.get((size_t)splits * M * N * sizeof(float))) {
+      BN = split_bn;
+      p.kb_per = per;
+      p.splits = splits;
+      p.part = static_cast<float*>(ws.p);
+    }
   }
   CUtensorMap ta, tb;
   st = bf16_map(enc, &ta, a, lda, K, M, 128);
@@ -628,11 +634,10 @@ oems_status oems_pk_relu_bwd(float* dy, const float* y, int64_t n, void* stream)
 }
 
 oems_status oems_pk_colsum(const float* dy, int64_t rows, int w, float* db, void* stream) {
-  if (rows >= 4096) {
-    const int parts = 148;
+  const int parts = 148;
+  Workspace ws(stream);
+  if (rows >= 4096 && ws.get((size_t)parts * w * sizeof(float))) {
     const long long per = (rows + parts - 1) / parts;
-    Workspace ws(stream);
-    PK_CUDA(ws.get((size_t)parts * w * sizeof(float)));
     float* part = static_cast<float*>(ws.p);
     if (w % 4 == 0 && aligned16(dy, dy))
       k_colsum_part<4><<<parts, 1024, 0, S(stream)>>>(dy, rows, w, per, part);

@@ -199,3 +199,19 @@ def test_graphs_of_both_parities_are_kept(child):
             e.run_batch(batch(n))
     assert F.fake_instantiated() == before
     """)
+
+
+def test_no_workspace_takes_the_forms_without(child):
+    """The GEMM's split sums and the column sum's parts are memory that the
+    one-part forms do not need."""
+    child("""
+    def calls():
+        a, b, c = (np.zeros(n, np.float32) for n in (128 * 4096, 640 * 4096, 128 * 640))
+        N.check(L.oems_tc_gemm_bf16(a.ctypes.data, 4096, b.ctypes.data, 4096, c.ctypes.data, 640, 128, 640, 4096, 0.0, None, None))
+        N.check(L.oems_pk_colsum(a.ctypes.data, 4096, 128, c.ctypes.data, None))
+        return [launched(k) for k in ("k_gemm_tc", "k_gemm_sum", "k_colsum_part", "k_colsumEPK")]
+    assert calls() == [1, 1, 1, 0]
+    knob("fail_pool_from", 0)
+    launched("", True)
+    assert calls() == [1, 0, 0, 1]
+    """)

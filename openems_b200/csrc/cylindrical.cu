@@ -56,8 +56,15 @@ oems_status cfail(oems_status st, const std::string& m) {
 // Row form: blocks of 256 threads, a z part of a row (a multiple of 32 cells,
 // as even as the row divides) times as many rows as fill the block.  Blocks of
 // 128 cells of one row left 37% of the lanes idle at 160 cells a row.
+// It is taken by rows of 128 cells and more and by shorter ones that fill
+// their warps; the rest keep the flat form, whose lanes are all at work (us a
+// step, flat / rows: 200 x 200 x 33 24.0 / 38.6, x 65 61.1 / 76.4, x 100 96.3
+// / 106.5; x 32 24.3 / 20.7, x 64 59.2 / 54.0, x 96 92.4 / 87.7, x 160 151 /
+// 137; 120 x 144 x 96 27.8 / 28.4, the one multiple of 32 where flat was as
+// good).
 constexpr int kCylRowThreads = 256;
-constexpr unsigned kCylRowMinZ = 24;  // shorter z rows use the flat form
+constexpr unsigned kCylRowMinZ = 128;
+inline bool cyl_rows(long long nz) { return nz >= kCylRowMinZ || nz % 32 == 0; }
 
 struct CylArgs {
   float* e[3];
@@ -106,7 +113,7 @@ __device__ __forceinline__ void current_cell(const CylArgs& a, unsigned i, unsig
   a.h[2][q] = __fadd_rn(a.h[2][q], __fmul_rn(__ldg(a.co[2] + q), c_z));
 }
 
-// Flat form: one thread per cell over the whole array (short z rows).
+// Flat form: one thread per cell over the whole array.
 template <bool kVoltage>
 __global__ void __launch_bounds__(256) k_cyl_flat(const CylArgs a) {
   const unsigned n = a.nr * a.na * a.nz;
@@ -231,7 +238,7 @@ static oems_status cyl_launch(oems_cyl_engine* en, uint64_t steps) {
   Dev g(en->device);
   const CylArgs v = args(en, true), c = args(en, false);
   const int gn = grid_of(en->n), gr = grid_of(en->na * en->nz);
-  const bool rows = (unsigned)en->nz >= kCylRowMinZ;
+  const bool rows = cyl_rows(en->nz);
   const long long parts = (en->nz + kCylRowThreads - 1) / kCylRowThreads;
   const long long bz = std::max<long long>(32, (((en->nz + parts - 1) / parts) + 31) / 32 * 32);
   const dim3 brow((unsigned)bz, (unsigned)std::max<long long>(1, kCylRowThreads / bz));

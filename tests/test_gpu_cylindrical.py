@@ -25,11 +25,18 @@ GRIDS = {
     "r0": ([i * 0.0005 for i in range(21)], [j * math.pi / 12 for j in range(25)], [k * 0.0005 for k in range(31)]),
     "open": (list(0.01 + 0.0004 * np.arange(17) ** 1.2), [0.0, 0.1, 0.25, 0.4, 0.5, 0.62, 0.8],
              [0.0, 0.001, 0.003, 0.004, 0.006, 0.0065, 0.008]),
-    # z rows of 128 cells or more take the row-tiled kernels (130: a ragged tail block)
+    # the grids above take the flat kernels; z rows of 128 cells or more and
+    # multiples of 32 below that the row kernels (130: a ragged tail block;
+    # 32 and 96: several rows a block, a last block of fewer)
     "rows": (list(np.linspace(0.005, 0.013, 9)), [j * 2 * math.pi / 12 for j in range(13)],
              list(np.linspace(0.0, 0.032, 161))),
     "rows_r0_open": ([i * 0.0005 for i in range(9)], [0.0, 0.2, 0.4, 0.6, 0.8, 1.0, 1.2],
                      list(np.linspace(0.0, 0.026, 131))),
+    "rows_32_closed": (list(np.linspace(0.005, 0.010, 6)), [j * 2 * math.pi / 11 for j in range(12)],
+                       list(np.linspace(0.0, 0.016, 33))),
+    "rows_96_r0": ([i * 0.0005 for i in range(8)], [j * math.pi / 7 for j in range(15)], list(np.linspace(0.0, 0.048, 97))),
+    "flat_127": (list(np.linspace(0.005, 0.009, 5)), [j * 2 * math.pi / 9 for j in range(10)],
+                 list(np.linspace(0.0, 0.0635, 128))),
 }
 
 

@@ -215,3 +215,18 @@ def test_no_workspace_takes_the_forms_without(child):
     launched("", True)
     assert calls() == [1, 0, 0, 1]
     """)
+
+
+@pytest.mark.parametrize("nz,rows", [(24, False), (31, False), (32, True), (33, False), (38, False), (64, True), (65, False),
+                                     (96, True), (106, False), (127, False), (128, True), (129, True), (160, True)])
+def test_cylindrical_form(child, nz, rows):
+    """The row form leaves lanes idle in short rows that do not fill their
+    warps: up to 1.6 times as long as the flat form."""
+    child(f"""
+    from openems_b200.cylindrical import CylindricalEngine, CylindricalGrid, CylindricalOperator
+    g = CylindricalGrid.uniform(0.005, 0.015, 5, 8, 0.0, 0.01, {nz})
+    assert g.dimensions()[2] == {nz}
+    with CylindricalEngine(CylindricalOperator(g, 1e-13)) as eng:
+        eng.step(2)
+    assert (launched("k_cyl_rows") > 0) == {rows} and (launched("k_cyl_flat") > 0) != {rows}
+    """)

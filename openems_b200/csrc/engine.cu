@@ -19,6 +19,7 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 
@@ -2313,128 +2314,189 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
 }
 
 // A stream, two events and two pinned buffers of one host thread's copies.
-// At most kMaxLanes a device are kept between calls (64 MB of pinned memory);
-// oems_release_cached_memory gives them back.
-constexpr size_t kPiece = (size_t)4 << 20;
+// At most kMaxLanes a device exist at a time (8 MB of pinned memory); they are
+// kept between calls and given back by oems_release_cached_memory.  Calls that
+// find them all in use wait for some: buffers made and dropped per call
+// (cudaFreeHost waits for the device) took four threads' reads of 50 MB from 18
+// ms to 250 and more.  Larger buffers gain little where the destination's pages
+// are new, as large arrays' are (744 MB in 49 ms with these, 42 with 4 MB).
+constexpr size_t kPiece = (size_t)512 << 10;
 constexpr size_t kMaxLanes = 8;
 struct CopyLane {
   cudaStream_t s = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  void* buf[2] = {nullptr, nullptr};
+  char* buf[2] = {nullptr, nullptr};
   cudaError_t make() {
     cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-    for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
-      e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
-      if (e == cudaSuccess) e = cudaMallocHost(&buf[k], kPiece);
-    }
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming);
+    void* p = nullptr;
+    if (e == cudaSuccess) e = cudaMallocHost(&p, 2 * kPiece);
+    buf[0] = static_cast<char*>(p);
+    buf[1] = buf[0] + kPiece;
     return e;
   }
   void drop() {
-    for (int k = 0; k < 2; ++k) {
-      if (buf[k]) cudaFreeHost(buf[k]);
-      if (ev[k]) cudaEventDestroy(ev[k]);
-    }
+    if (buf[0]) cudaFreeHost(buf[0]);
+    for (cudaEvent_t e : ev)
+      if (e) cudaEventDestroy(e);
     if (s) cudaStreamDestroy(s);
     *this = CopyLane{};
   }
 };
+// A lane's pinned memory takes 0.5 ms and more to make (tens of ms where other
+// threads fault pages in meanwhile), a small copy's whole gain, so lanes are
+// made as they are paid for: a call adds a 16th of its bytes to the credit, and
+// a process' first lane is on the house.  Eight lanes of 8 MB made on first use
+// took the first read of 2.5 MB from 3.2 to 43 ms, of 98 MB from 25 to 54.
 struct LanePool {
   std::mutex mu;
-  std::vector<CopyLane> free[kMaxDevices];
+  std::condition_variable cv;
+  std::vector<CopyLane> free;
+  size_t made = 0;  // free and in use
+  size_t credit = 0;
+  LanePool() { free.reserve(kMaxLanes); }
 };
-static LanePool& lane_pool() {
-  static LanePool p;
-  return p;
-}
-static cudaError_t lane_get(int device, CopyLane* out) {
-  LanePool& p = lane_pool();
-  {
-    std::lock_guard<std::mutex> lk(p.mu);
-    if (device < kMaxDevices && !p.free[device].empty()) {
-      *out = p.free[device].back();
-      p.free[device].pop_back();
-      return cudaSuccess;
-    }
-  }
-  return out->make();
+static LanePool& lane_pool(int device) {
+  static LanePool p[kMaxDevices];
+  return p[device];
 }
 static void lane_put(int device, CopyLane lane, bool ok) {
-  LanePool& p = lane_pool();
+  LanePool& p = lane_pool(device);
+  if (!ok) lane.drop();
   {
     std::lock_guard<std::mutex> lk(p.mu);
-    if (ok && device < kMaxDevices && p.free[device].size() < kMaxLanes) {
-      p.free[device].push_back(lane);
-      return;
+    if (ok)
+      p.free.push_back(lane);  // (reserved)
+    else
+      --p.made;
+  }
+  p.cv.notify_all();
+}
+// Up to `want` lanes for a copy of `total` bytes; while others use most of the
+// lanes, waits for half of `want`.  None: no pinned memory is to be had.
+static std::vector<CopyLane> lanes_get(int device, size_t want, size_t total) {
+  LanePool& p = lane_pool(device);
+  std::vector<CopyLane> got;
+  got.reserve(want);
+  size_t fresh = 0;
+  {
+    std::unique_lock<std::mutex> lk(p.mu);
+    p.credit = std::min(p.credit + total / 16, 2 * kMaxLanes * kPiece);
+    p.cv.wait(lk, [&] {
+      const size_t can = p.free.size() + std::min(p.credit / (2 * kPiece), kMaxLanes - p.made);
+      return p.free.size() == p.made || can >= std::min({(want + 1) / 2, kMaxLanes / 2, p.made});
+    });
+    while (got.size() < want && !p.free.empty()) {
+      got.push_back(p.free.back());
+      p.free.pop_back();
+    }
+    for (; got.size() + fresh < want && p.made < kMaxLanes && (p.credit >= 2 * kPiece || p.made == 0); ++fresh, ++p.made)
+      p.credit -= std::min(p.credit, 2 * kPiece);
+  }
+  for (; fresh > 0; --fresh) {
+    CopyLane l;
+    if (l.make() == cudaSuccess) {
+      got.push_back(l);
+    } else {
+      cudaGetLastError();
+      lane_put(device, l, false);
     }
   }
-  lane.drop();
+  return got;
+}
+
+static cudaError_t copy_out_plain(float* const* dst, const float* const* src, int count, size_t rows, size_t width,
+                                  size_t pitch, cudaStream_t after) {
+  for (int c = 0; c < count; ++c) {
+    const cudaError_t e =
+        width == pitch
+            ? cudaMemcpyAsync(dst[c], src[c], rows * width * sizeof(float), cudaMemcpyDeviceToHost, after)
+            : cudaMemcpy2DAsync(dst[c], width * sizeof(float), src[c], pitch * sizeof(float), width * sizeof(float),
+                                rows, cudaMemcpyDeviceToHost, after);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaStreamSynchronize(after);
 }
 
 // Device arrays to pageable host memory.  The driver's own staging of such a
 // copy runs on one thread and takes the destination's page faults there: 7
 // GB/s, and 1.7 GB/s into memory no one has touched.  Here up to eight host
 // threads each copy pieces through two pinned buffers: while one piece is on
-// the bus, others are moved to their place (400 MB in 16 ms where it took 58
-// to 85; 744 MB in 39 ms instead of 275).  Pieces are whole padded rows (pitch
-// elements, of which the first width go to the host), at most 4 MB, about 16
-// to a copy; below 1 MB the threads cost more than they save.
+// the bus, others are moved to their place.  Pieces are whole padded rows
+// (pitch elements, of which the first width go to the host).  Into warm / fresh
+// pages, plain -> pieces: 20 MB 1.3 / 8.8 -> 0.7 / 1.8 ms, 250 MB 14.7 / 110 ->
+// 8 / 16 ms.  Below kThreads bytes the calling thread does it all: others, on
+// cores idle while the steps ran, take 0.1 to 0.5 ms to come to work (60 steps
+// of a 2.5 MB grid with its read-back took 0.83 ms plain, 0.96 with four
+// threads, 0.78 with one).  One lane: 2.5 MB 277 -> 212 us warm, 1.2 -> 0.7 ms
+// fresh; 6.9 MB 607 -> 577 us, 3.2 -> 1.9 ms; 15 MB 1.05 -> 0.98, 6.7 -> 4.1 ms;
+// from 20 MB on it is the plain copy's equal on warm pages.  Where no pinned
+// memory (or thread) is to be had the copy goes on with fewer, down to the
+// plain form.
+constexpr size_t kThreads = (size_t)16 << 20;
 cudaError_t copy_out(int device, float* const* dst, const float* const* src, int count, size_t rows, size_t width,
                      size_t pitch, cudaStream_t after) {
   const size_t row = pitch * sizeof(float), total = (size_t)count * rows * row;
-  if (total < ((size_t)1 << 20) || row > kPiece) {
-    for (int c = 0; c < count; ++c) {
-      const cudaError_t e = cudaMemcpy2DAsync(dst[c], width * sizeof(float), src[c], pitch * sizeof(float),
-                                              width * sizeof(float), rows, cudaMemcpyDeviceToHost, after);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaStreamSynchronize(after);
-  }
+  if (total < ((size_t)1 << 20) || row > kPiece || device < 0 || device >= kMaxDevices)
+    return copy_out_plain(dst, src, count, rows, width, pitch, after);
   cudaError_t err = cudaStreamSynchronize(after);
   if (err != cudaSuccess) return err;
-  const size_t per = std::max<size_t>(1, std::min(kPiece, std::max<size_t>(total / 16, 256 << 10)) / row);  // rows
-  const size_t pieces_each = (rows + per - 1) / per, pieces = pieces_each * count;
-  std::atomic<size_t> next{0};
+  std::vector<CopyLane> lanes = lanes_get(device, total < kThreads ? 1 : kMaxLanes, total);
+  if (lanes.empty()) return copy_out_plain(dst, src, count, rows, width, pitch, after);
+  // rows of a piece: four pieces at least to a lane alone, two to each of several
+  const size_t per = std::max<size_t>(1, std::min(kPiece, total / (lanes.size() > 1 ? 2 * lanes.size() : 4)) / row);
+  const size_t all = rows * (size_t)count;
+  std::atomic<size_t> next{0};  // next row of all arrays' to be taken
   std::atomic<int> failed{cudaSuccess};
-  auto work = [&] {
+  auto work = [&](CopyLane lane) {
     DeviceGuard guard(device);
-    CopyLane lane;
-    cudaError_t e = lane_get(device, &lane);
-    size_t piece[2] = {pieces, pieces};  // in flight in each buffer
+    cudaError_t e = cudaSuccess;
+    size_t from[2] = {0, 0}, n[2] = {0, 0};  // rows in flight
     auto land = [&](int k) {
-      if (piece[k] >= pieces || e != cudaSuccess) return;
+      if (!n[k] || e != cudaSuccess) return;
       if ((e = cudaEventSynchronize(lane.ev[k])) != cudaSuccess) return;
-      const size_t c = piece[k] / pieces_each, r0 = (piece[k] - c * pieces_each) * per, n = std::min(per, rows - r0);
-      const float* from = static_cast<const float*>(lane.buf[k]);
-      float* to = dst[c] + r0 * width;
+      const size_t c = from[k] / rows;
+      const float* in = reinterpret_cast<const float*>(lane.buf[k]);
+      float* to = dst[c] + (from[k] - c * rows) * width;
       if (width == pitch)
-        std::memcpy(to, from, n * width * sizeof(float));
+        std::memcpy(to, in, n[k] * width * sizeof(float));
       else
-        for (size_t r = 0; r < n; ++r) std::memcpy(to + r * width, from + r * pitch, width * sizeof(float));
-      piece[k] = pieces;
+        for (size_t r = 0; r < n[k]; ++r) std::memcpy(to + r * width, in + r * pitch, width * sizeof(float));
+      n[k] = 0;
     };
     for (int k = 0; e == cudaSuccess && failed.load() == cudaSuccess; k ^= 1) {
       land(k);
-      const size_t q = next.fetch_add(1);
-      if (q >= pieces || e != cudaSuccess) break;
-      const size_t c = q / pieces_each, r0 = (q - c * pieces_each) * per, n = std::min(per, rows - r0);
-      e = cudaMemcpyAsync(lane.buf[k], src[c] + r0 * pitch, n * row, cudaMemcpyDeviceToHost, lane.s);
+      if (e != cudaSuccess) break;
+      size_t q = next.load(), m = 0;
+      do {
+        if (q >= all) break;
+        m = std::min(per, rows - q % rows);
+      } while (!next.compare_exchange_weak(q, q + m));
+      if (q >= all) break;
+      const size_t c = q / rows;
+      e = cudaMemcpyAsync(lane.buf[k], src[c] + (q - c * rows) * pitch, m * row, cudaMemcpyDeviceToHost, lane.s);
       if (e == cudaSuccess) e = cudaEventRecord(lane.ev[k], lane.s);
-      piece[k] = q;
+      from[k] = q;
+      n[k] = m;
     }
     land(0);
     land(1);
-    if (lane.s) cudaStreamSynchronize(lane.s);  // nothing of ours is in flight before the buffers go back
+    cudaStreamSynchronize(lane.s);  // nothing of ours is in flight before the buffers go back
     lane_put(device, lane, e == cudaSuccess);
     if (e != cudaSuccess) failed.store(e);
   };
   std::vector<std::thread> t;
-  const size_t most = std::min<size_t>({8, pieces, std::max(1u, std::thread::hardware_concurrency())});
-  try {
-    t.reserve(most);
-    while (t.size() + 1 < most) t.emplace_back(work);
-  } catch (const std::exception&) {  // no more threads: the ones there do the work
+  t.reserve(kMaxLanes);
+  while (lanes.size() > 1) {
+    try {
+      t.emplace_back(work, lanes.back());
+    } catch (const std::exception&) {  // no more threads: the ones there do the work
+      for (; lanes.size() > 1; lanes.pop_back()) lane_put(device, lanes.back(), true);
+      break;
+    }
+    lanes.pop_back();
   }
-  work();
+  work(lanes[0]);
   for (std::thread& x : t) x.join();
   return static_cast<cudaError_t>(failed.load());
 }
@@ -4018,8 +4080,11 @@ oems_status oems_release_cached_memory(int32_t device) {
   }
   std::vector<CopyLane> lanes;
   if (dev >= 0 && dev < kMaxDevices) {
-    std::lock_guard<std::mutex> lk(lane_pool().mu);
-    lanes.swap(lane_pool().free[dev]);
+    LanePool& p = lane_pool(dev);
+    std::lock_guard<std::mutex> lk(p.mu);
+    lanes = p.free;
+    p.free.clear();
+    p.made -= lanes.size();
   }
   for (CopyLane& l : lanes) l.drop();
   std::multimap<size_t, void*> bufs;

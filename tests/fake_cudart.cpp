@@ -48,7 +48,7 @@ std::map<void*, Block>& blocks() {
   static std::map<void*, Block> m;
   return m;
 }
-long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, instantiated = 0;
+long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, instantiated = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local int capturing = 0;
 
@@ -125,7 +125,8 @@ long long fake_launched(const char* part, int reset) {
   return n;
 }
 long long fake_pool_used() { return pooled; }
-long long fake_pinned() { return pinned; }
+long long fake_pinned() { return pinned; }  // bytes now
+long long fake_pins() { return pins; }      // calls so far
 long long fake_instantiated() { return instantiated; }
 
 cudaError_t cudaMalloc(void** p, size_t n) { return alloc(p, n, false); }
@@ -135,13 +136,21 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return give(p); }
 cudaError_t cudaMallocHost(void** p, size_t n) {
   if (refuse("fail_host", "pass_host")) return ret(cudaErrorMemoryAllocation);
   std::lock_guard<std::recursive_mutex> lk(mu);
-  ++pinned;
-  return (*p = std::malloc(n)) ? cudaSuccess : ret(cudaErrorMemoryAllocation);
+  char* q = static_cast<char*>(std::malloc(n + 64));
+  if (!q) return ret(cudaErrorMemoryAllocation);
+  std::memcpy(q, &n, sizeof(n));
+  pinned += (long long)n;
+  ++pins;
+  *p = q + 64;
+  return cudaSuccess;
 }
 cudaError_t cudaFreeHost(void* p) {
   std::lock_guard<std::recursive_mutex> lk(mu);
-  --pinned;
-  std::free(p);
+  size_t n = 0;
+  char* q = static_cast<char*>(p) - 64;
+  std::memcpy(&n, q, sizeof(n));
+  pinned -= (long long)n;
+  std::free(q);
   return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {

@@ -22,7 +22,7 @@ import openems_b200._native as N
 N.LIB_PATH = %r
 import openems_b200 as oe
 L, F = N.lib(), ctypes.CDLL(N.LIB_PATH)
-for f in ("fake_launched", "fake_pool_used", "fake_pinned", "fake_instantiated"):
+for f in ("fake_launched", "fake_pool_used", "fake_pinned", "fake_pins", "fake_instantiated"):
     getattr(F, f).restype = ctypes.c_longlong
 F.fake_set.argtypes = [ctypes.c_char_p, ctypes.c_longlong]
 
@@ -229,4 +229,49 @@ def test_cylindrical_form(child, nz, rows):
     with CylindricalEngine(CylindricalOperator(g, 1e-13)) as eng:
         eng.step(2)
     assert (launched("k_cyl_rows") > 0) == {rows} and (launched("k_cyl_flat") > 0) != {rows}
+    """)
+
+
+# no pinned memory; some of the lanes; none for the second call's larger pieces
+@pytest.mark.parametrize("passed", [0, 1, 3])
+@pytest.mark.parametrize("dims", [(60, 61, 62), (100, 120, 127)])  # one lane; several
+def test_refused_pinned_memory_does_not_fail_a_read(child, passed, dims):
+    child(f"""
+    e = engine({dims})
+    f = np.random.default_rng(0).standard_normal((2, 3) + {dims}, dtype=np.float32)
+    e.write_fields(f[0], f[1])
+    knob("pass_host", {passed}), knob("fail_host", -1)
+    for _ in range(4):
+        got = e.read_fields()
+        assert np.array_equal(got[0], f[0]) and np.array_equal(got[1], f[1])
+    """)
+
+
+def test_concurrent_reads_share_the_pinned_buffers(child):
+    """Made once, whatever the number of callers, and bounded."""
+    child("""
+    from concurrent.futures import ThreadPoolExecutor
+    es, fs = [], []
+    for k in range(6):
+        es.append(engine((100, 120, 121 + k)))
+        fs.append(np.random.default_rng(k).standard_normal((2, 3, 100, 120, 121 + k), dtype=np.float32))
+        es[k].write_fields(fs[k][0], fs[k][1])
+    for _ in range(30):  # (the buffers grow with what has been copied)
+        es[0].read_fields()
+    before = F.fake_pins()
+    with ThreadPoolExecutor(6) as pool:
+        for _ in range(20):
+            for got, f in zip(pool.map(lambda e: e.read_fields(), es), fs):
+                assert np.array_equal(got[0], f[0]) and np.array_equal(got[1], f[1])
+    assert F.fake_pins() - before <= 16 and F.fake_pinned() <= 65 << 20
+    L.oems_release_cached_memory(0)
+    assert F.fake_pinned() < 1 << 20
+    """)
+
+
+def test_a_small_first_read_pins_little(child):
+    """Pinned memory takes longer to make than a read of a few MB."""
+    child("""
+    engine((40, 40, 65)).read_fields()
+    assert F.fake_pinned() <= 1 << 20
     """)

@@ -581,11 +581,11 @@ struct FusedPlan {
   double cost = 0.0;
 };
 struct FusedKey {
-  int dev, nx, ny, nz, id_bytes, ntable, mode;
+  int dev, nx, ny, nz, id_bytes, table_room, mode;
   std::array<int, 6> layers;  // of the CPML: a plan's boxes follow its slabs
   bool operator<(const FusedKey& o) const {
-    return std::tie(dev, nx, ny, nz, id_bytes, ntable, mode, layers) <
-           std::tie(o.dev, o.nx, o.ny, o.nz, o.id_bytes, o.ntable, o.mode, o.layers);
+    return std::tie(dev, nx, ny, nz, id_bytes, table_room, mode, layers) <
+           std::tie(o.dev, o.nx, o.ny, o.nz, o.id_bytes, o.table_room, o.mode, o.layers);
   }
 };
 struct FusedHost {

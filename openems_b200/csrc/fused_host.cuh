@@ -352,11 +352,21 @@ static double fused_cost(const FusedPlan& p, int sms, const int (&occ)[2], std::
 // when launched back to back, and a fifth slower inside a graph.)
 constexpr long long kFusedSmall = 3000000;
 
+// Sets of the table a CTA's shared memory has room for: plans, and the tuning
+// they take, are shared by the grids of one size whose numbers of sets round up
+// to the same (a new scene of boxes is rarely of the same number).
+static int fused_table_room(const oems_engine* en) {
+  if (en->fus.id_bytes != 1) return 0;
+  int n = 32;
+  while (n < en->fus.ntable) n *= 2;
+  return n;
+}
+
 // Shapes for passes of `steps`, best first by the model.
 static std::vector<FusedPlan> fused_shapes(const oems_engine* en, int steps, int sms, size_t smem_cta,
                                            size_t smem_sm) {
   const int prof = fused_prof_floats(en);
-  const int tab = en->fus.id_bytes == 1 ? en->fus.ntable * 12 : 0;
+  const int tab = fused_table_room(en) * 12;
   std::vector<FusedPlan> all;
   std::vector<double> heap;
   struct Cta {
@@ -552,7 +562,7 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
   const bool time_it = !(en->flags & OEMS_ENGINE_NO_AUTOTUNE);
   std::array<int, 6> layers{};
   if (en->cpml.on) std::copy(en->cpml.args.L, en->cpml.args.L + 6, layers.begin());
-  const FusedKey key{en->device, en->nx, en->ny, en->nz, F.id_bytes, F.id_bytes == 1 ? F.ntable : 0,
+  const FusedKey key{en->device, en->nx, en->ny, en->nz, F.id_bytes, fused_table_room(en),
                      (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0), layers};
   std::vector<FusedPlan> plans;
   en->tune_report.clear();

@@ -275,3 +275,24 @@ def test_a_small_first_read_pins_little(child):
     engine((40, 40, 65)).read_fields()
     assert F.fake_pinned() <= 1 << 20
     """)
+
+
+def test_scenes_of_other_materials_share_their_plans(child):
+    """A plan was found by up to 33 timings again whenever the number of
+    distinct coefficient sets was another."""
+    child("""
+    def one(n):
+        op = oe.Operator(oe.Grid.uniform(30, 31, 32, 1e-3), oe.BoundaryConditions.all_pec())
+        for k in range(n):
+            op.set_material(2.0 + k, 1.0, 0.0, 0.0, (k, k + 1, 0, 31, 0, 32))
+        e = oe.Engine(op, compressed=True)
+        e.add_cpml(oe.CpmlBoundaries(layers=(4,) * 6))
+        launched("", True)
+        e.run_batch(batch(5))
+        return launched("k_fused"), len(e.tune_report())
+    first = one(2)
+    assert first[0] > 200 and first[1] > 20
+    for n in (5, 9, 20):
+        again = one(n)
+        assert again[0] < 20 and again[1] == first[1]
+    """)

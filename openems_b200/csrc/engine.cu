@@ -591,7 +591,7 @@ struct FusedKey {
 struct FusedHost {
   int state = 0;      // 0 not looked at, 1 prepared, -1 not for this engine
   bool use = false;   // this batch runs as fused passes
-  bool tuned = false, tuned_pack = false;
+  int tuned = 0, tuned_pack = 0;  // longest passes plans were found for (0: none yet)
   int parity = 0;     // which of the two buffer sets is current
   DevBuf<char> alt;   // the buffers the next pass writes
   DevBuf<float> psi;
@@ -2129,7 +2129,7 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
   en->last_launches = 0;
   bool fused = false;
   OEMS_TRY(fused_ready(en, &fused));
-  if (fused && !en->fus.tuned) OEMS_TRY(fused_tune(en, &fused));
+  if (fused && en->fus.tuned != fused_max_steps(en)) OEMS_TRY(fused_tune(en, &fused));
   if (fused != en->fus.use || en->fus.packed) en->graph_epoch++;
   en->fus.use = fused;
   en->fus.packed = false;
@@ -2753,7 +2753,7 @@ static oems_status add_cpml(oems_engine* en, const oems_cpml_desc* d) {
   en->cpml.on = true;
   en->cpml.desc = *d;
   en->tuned = false;  // the CPML kernels get their own launch shape
-  en->fus.tuned = en->fus.tuned_pack = false;
+  en->fus.tuned = en->fus.tuned_pack = 0;
   LaunchShape s = en->shape;
   OEMS_TRY(size_grid(en, s));
   apply_shape(en, s);

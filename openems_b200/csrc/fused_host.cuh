@@ -542,9 +542,9 @@ static std::map<FusedKey, FusedTuned>& fused_cache() {
   return m;
 }
 
-// Tile shapes of the one- and two-step passes: the model's best, or (with
-// the autotuner) the fastest of its first few on the engine's own state,
-// which a pass only reads.  *ok: false where a CTA's shared memory takes no
+// Tile shapes of the passes the engine may take (fused_max_steps): the model's
+// best, or (with the autotuner) the fastest of its first few on the engine's
+// own state, which a pass only reads.  *ok: false where a CTA's shared memory takes no
 // tile at all (CPML profiles of thousands of layers): the engine then keeps
 // the separate kernels.
 static oems_status fused_tune(oems_engine* en, bool* ok) {
@@ -554,7 +554,8 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
   OEMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, en->device));
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, en->device));
-  for (int steps = 1; steps <= 2; ++steps)
+  const int longest = fused_max_steps(en);
+  for (int steps = 1; steps <= longest; ++steps)
     for (bool cpml : {false, true})
       OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
@@ -563,7 +564,7 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
   std::array<int, 6> layers{};
   if (en->cpml.on) std::copy(en->cpml.args.L, en->cpml.args.L + 6, layers.begin());
   const FusedKey key{en->device, en->nx, en->ny, en->nz, F.id_bytes, fused_table_room(en),
-                     (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0), layers};
+                     (en->cpml.on ? 1 : 0) | en->storage << 1 | (time_it ? 8 : 0) | longest << 4, layers};
   std::vector<FusedPlan> plans;
   en->tune_report.clear();
   {
@@ -575,22 +576,20 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
     }
   }
   const bool cached = !plans.empty();
-  for (int steps = 1; steps <= 2; ++steps) {
+  for (int steps = 1; steps <= longest; ++steps) {
     std::vector<FusedPlan> c;
-    const bool have = cached && plans[steps - 1].nbox > 0;
-    if (have)
+    if (cached)
       c.push_back(plans[steps - 1]);
     else
       c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
     if (c.empty()) {
-      if (steps > fused_max_steps(en)) continue;
       F.state = -1;
       fused_release(en);
       return OEMS_OK;
     }
-    // one-step passes only finish odd spans unless an extension needs them
+    // shorter passes only finish odd spans
     const bool small = en->ncells_padded < kFusedSmall;
-    const size_t most = have || !time_it ? 1 : steps != fused_max_steps(en) ? 3 : small ? 30 : 12;
+    const size_t most = cached || !time_it ? 1 : steps != longest ? 3 : small ? 30 : 12;
     if (c.size() > most) c.resize(most);
     FusedPlan best = c[0];
     if (c.size() > 1) {
@@ -624,7 +623,8 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
     std::lock_guard<std::mutex> lock(tune_mutex());
     fused_cache()[key] = FusedTuned{{F.plan[0], F.plan[1]}, en->tune_report};
   }
-  F.tuned = *ok = true;
+  F.tuned = longest;
+  *ok = true;
   en->graph_epoch++;
   return OEMS_OK;
 }
@@ -634,7 +634,7 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
 static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
   FusedHost& F = en->fus;
   const int most = fused_max_steps(en);
-  if (F.pack_sms == sms && F.tuned_pack) {
+  if (F.pack_sms == sms && F.tuned_pack == most) {
     *ok = F.pack_plan[most - 1].nbox > 0;
     return OEMS_OK;
   }
@@ -643,7 +643,7 @@ static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
   int smem_cta = 0, smem_sm = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, en->device));
-  for (int steps = 1; steps <= 2; ++steps) {
+  for (int steps = 1; steps <= most; ++steps) {
     for (bool cpml : {false, true})
       OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
@@ -653,7 +653,7 @@ static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
   }
   *ok = F.pack_plan[most - 1].nbox > 0;
   F.pack_sms = sms;
-  F.tuned_pack = true;
+  F.tuned_pack = most;
   en->graph_epoch++;
   return OEMS_OK;
 }

@@ -296,3 +296,23 @@ def test_scenes_of_other_materials_share_their_plans(child):
         again = one(n)
         assert again[0] < 20 and again[1] == first[1]
     """)
+
+
+def test_plans_of_one_step_engines_are_searched(child):
+    """A Mur engine of a grid that a plain engine ran before tunes its
+    one-step passes as if it had been the first, and so does an engine that is
+    given a recorder later."""
+    child("""
+    def tried(e):
+        e.run_batch(batch(4))
+        return sorted(r["extra"] % 10 for r in e.tune_report())
+    plain = engine((30, 31, 32))
+    assert tried(plain).count(2) > 10 and launched("k_fused") > 0
+    mur = engine((30, 31, 32))
+    mur.add_mur(oe.MurAbcConfig.all(1))
+    assert tried(mur).count(1) > 10 and tried(mur).count(2) == 0
+    late = engine((30, 31, 33))
+    assert tried(late).count(2) > 10
+    oe.fdtd.Nf2ffBox(late, (4, 4, 4), (15, 15, 15), [1e9])
+    assert tried(late).count(1) > 10 and fused(late) and late.launch_info()["stages"] == 1
+    """)

@@ -53,9 +53,9 @@ static void fused_release(oems_engine* en) {
 }
 
 // Ids and table of the distinct coefficient sets of a full-array engine, by
-// two kernels over the arrays.  More than 65,536 sets, two sets with one hash
-// or no room for the tables: the engine keeps its full arrays and the
-// register kernels.
+// two kernels over the arrays.  More than 65,536 sets or two sets with one hash:
+// the engine keeps its full arrays and the register kernels for good; no room
+// for the tables: for now.
 static oems_status fused_ids(oems_engine* en, bool* ok) {
   FusedHost& F = en->fus;
   *ok = false;
@@ -93,7 +93,10 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   int n[2];
   OEMS_CUDA(cudaMemcpyAsync(n, count.p, sizeof(n), cudaMemcpyDeviceToHost, en->stream));
   OEMS_CUDA(cudaStreamSynchronize(en->stream));
-  if (n[1] || n[0] > kCoefMax) return OEMS_OK;
+  if (n[1] || n[0] > kCoefMax) {
+    F.state = -1;
+    return OEMS_OK;
+  }
   DevBuf<long long> first;
   if (!got_room(first.ensure(n[0]))) return OEMS_OK;
   k_coef_first<<<blocks_for(n[0], 256), 256, 0, en->stream>>>(list.p, rep.p, n[0], first.p);
@@ -129,31 +132,57 @@ static oems_status fused_ids(oems_engine* en, bool* ok) {
   OEMS_CUDA(cudaGetLastError());
   OEMS_CUDA(cudaMemcpyAsync(n, count.p, sizeof(n), cudaMemcpyDeviceToHost, en->stream));
   OEMS_CUDA(cudaStreamSynchronize(en->stream));
-  if (n[1]) return OEMS_OK;
+  if (n[1]) {
+    F.state = -1;
+    return OEMS_OK;
+  }
   F.ids = F.own_ids.p;
   F.table = F.own_table.p;
   *ok = true;
   return OEMS_OK;
 }
 
+// Whether the engine's kind allows fused passes.  Kernels asked for by name,
+// TF/SF planes and the UPML (which change fields between the H and E halves)
+// keep the separate updates.
+static bool fused_kind(const oems_engine* en) {
+  const uint32_t forced = OEMS_ENGINE_STAGED_KERNELS | OEMS_ENGINE_REGISTER_KERNELS | OEMS_ENGINE_SPLIT_KERNELS |
+                          OEMS_ENGINE_ZSPLIT_KERNELS | OEMS_ENGINE_PIPE_KERNELS;
+  return !((en->flags & forced) || en->tfsf.on || en->upml.on || en->fus.state < 0 ||
+           (long long)en->ny * en->g.nzq > INT32_MAX / 2);
+}
+
+// Device memory that an engine's buffers may still take: the driver's free
+// bytes and the freed blocks that the pool holds.
+static oems_status fused_free_bytes(const oems_engine* en, size_t* out) {
+  size_t total = 0;
+  OEMS_CUDA(cudaMemGetInfo(out, &total));
+  cudaMemPool_t pool = nullptr;
+  uint64_t held = 0, used = 0;
+  if (device_pool(en->device, false, &pool) == cudaSuccess && pool) {
+    OEMS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+    OEMS_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+    *out += held > used ? (size_t)(held - used) : 0;
+  }
+  return OEMS_OK;
+}
+
+// What the engine's second buffers are still to take; a quarter of the free
+// memory at most, or it keeps the separate kernels (until there is more).
+static size_t fused_need(const oems_engine* en) {
+  return en->fus.state > 0 ? 0 : en->field_bytes() + (en->id_bytes ? 0 : (size_t)en->ncells_padded);
+}
+
 // Whether this engine's batches run as fused passes; prepares ids and the
-// second buffers on first use.  Kernels asked for by name, TF/SF planes and
-// the UPML (which change fields between the H and E halves) keep the separate
-// updates, as do grids whose second buffers would take more than a quarter of
-// the free memory.
+// second buffers on first use.
 static oems_status fused_ready(oems_engine* en, bool* yes) {
   FusedHost& F = en->fus;
   *yes = false;
-  const uint32_t forced = OEMS_ENGINE_STAGED_KERNELS | OEMS_ENGINE_REGISTER_KERNELS | OEMS_ENGINE_SPLIT_KERNELS |
-                          OEMS_ENGINE_ZSPLIT_KERNELS | OEMS_ENGINE_PIPE_KERNELS;
-  if ((en->flags & forced) || en->tfsf.on || en->upml.on || F.state < 0) return OEMS_OK;
+  if (!fused_kind(en)) return OEMS_OK;
   if (F.state == 0) {
-    F.state = -1;
-    if ((long long)en->ny * en->g.nzq > INT32_MAX / 2) return OEMS_OK;
-    const size_t need = en->field_bytes() + (en->id_bytes ? 0 : (size_t)en->ncells_padded);
-    size_t free_b = 0, total_b = 0;
-    OEMS_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if (need > free_b / 4) return OEMS_OK;
+    size_t free_b = 0;
+    OEMS_TRY(fused_free_bytes(en, &free_b));
+    if (fused_need(en) > free_b / 4) return OEMS_OK;
     bool ok = false;
     OEMS_TRY(fused_ids(en, &ok));
     if (!ok || !got_room(F.alt.ensure(en->field_bytes()))) {
@@ -166,7 +195,7 @@ static oems_status fused_ready(oems_engine* en, bool* yes) {
   }
   if (en->cpml.on && F.psi.n != en->cpml.psi.n) {
     if (!got_room(F.psi.ensure(en->cpml.psi.n))) {
-      F.state = -1;
+      F.state = 0;
       fused_release(en);
       return OEMS_OK;
     }
@@ -634,11 +663,8 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
 static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
   FusedHost& F = en->fus;
   const int most = fused_max_steps(en);
-  if (F.pack_sms == sms && F.tuned_pack == most) {
-    *ok = F.pack_plan[most - 1].nbox > 0;
-    return OEMS_OK;
-  }
-  F.pack_plan[0] = F.pack_plan[1] = FusedPlan{};
+  *ok = F.pack_sms == sms && F.tuned_pack == most;
+  if (*ok) return OEMS_OK;
   if (en->cpml.on) side_stream(en);  // (not for the first time inside a capture)
   int smem_cta = 0, smem_sm = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&smem_cta, cudaDevAttrMaxSharedMemoryPerBlockOptin, en->device));
@@ -648,10 +674,14 @@ static oems_status fused_pack_tune(oems_engine* en, int sms, bool* ok) {
       OEMS_CUDA(cudaFuncSetAttribute((const void*)pick_fused(en, steps, cpml),
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_cta));
     const std::vector<FusedPlan> c = fused_shapes(en, steps, sms, smem_cta, smem_sm);
-    if (c.empty()) break;
+    if (c.empty()) {
+      F.state = -1;
+      fused_release(en);
+      return OEMS_OK;
+    }
     F.pack_plan[steps - 1] = c[0];
   }
-  *ok = F.pack_plan[most - 1].nbox > 0;
+  *ok = true;
   F.pack_sms = sms;
   F.tuned_pack = most;
   en->graph_epoch++;

@@ -316,3 +316,19 @@ def test_plans_of_one_step_engines_are_searched(child):
     oe.fdtd.Nf2ffBox(late, (4, 4, 4), (15, 15, 15), [1e9])
     assert tried(late).count(1) > 10 and fused(late) and late.launch_info()["stages"] == 1
     """)
+
+
+def test_memory_that_is_tight_once_is_not_held_against_an_engine(child):
+    """The quarter counts what the pool holds free, and is looked at again."""
+    child("""
+    mb = 24 * 64 ** 3 / 2.0 ** 20  # fields of an engine; coefficients are twice that
+    knob("capacity", int(12 * mb * 2 ** 20))
+    big = [engine((64, 64, 64), autotune=False) for _ in range(3)]
+    e = big[0]
+    e.run_batch(batch(4))
+    assert not fused(e)
+    big[2].close()  # to the pool, not to the driver
+    big[1].close()
+    e.run_batch(batch(4))
+    assert fused(e)
+    """)

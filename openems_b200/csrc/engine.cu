@@ -589,7 +589,7 @@ struct FusedKey {
   }
 };
 struct FusedHost {
-  int state = 0;      // 0 not looked at, 1 prepared, -1 not for this engine
+  int state = 0;      // 0 not prepared, 1 prepared, -1 not for this engine
   bool use = false;   // this batch runs as fused passes
   int tuned = 0, tuned_pack = 0;  // longest passes plans were found for (0: none yet)
   int parity = 0;     // which of the two buffer sets is current
@@ -4491,13 +4491,38 @@ static oems_status pack_fused(oems_pack* p, const std::vector<int>& part, bool* 
   if (p->shape_set) return OEMS_OK;  // a shape of the shared launches was asked for
   int sms = 0;
   OEMS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
+  // all of them or none: what was made for the first engines of a pack that
+  // cannot run fused goes back
   double cells = 0;
+  size_t free_b = 0, needs = 0;
   for (int i : part) {
-    EngineScope guard(p->en[i]);
+    if (!fused_kind(p->en[i])) return OEMS_OK;
+    needs += fused_need(p->en[i]);
+  }
+  if (needs > 0) OEMS_TRY(fused_free_bytes(p->en[part[0]], &free_b));
+  for (int i : part) {
+    const size_t need = fused_need(p->en[i]);
+    if (need > free_b / 4) return OEMS_OK;
+    free_b -= need;
+  }
+  std::vector<oems_engine*> made;
+  auto give_back = [&] {
+    for (oems_engine* en : made) {
+      EngineScope guard(en);
+      fused_release(en);
+      en->fus.state = std::min(en->fus.state, 0);
+    }
+  };
+  for (int i : part) {
+    oems_engine* en = p->en[i];
+    EngineScope guard(en);
     bool ok = false;
-    OEMS_TRY(fused_ready(p->en[i], &ok));
-    if (!ok) return OEMS_OK;
-    cells += (double)p->en[i]->ncells_padded;
+    const bool had = en->fus.state > 0;
+    const oems_status st = fused_ready(en, &ok);
+    if (!had && en->fus.state > 0) made.push_back(en);
+    if (!ok) give_back();
+    if (st != OEMS_OK || !ok) return st;
+    cells += (double)en->ncells_padded;
   }
   for (int i : part) {
     oems_engine* en = p->en[i];
@@ -4506,8 +4531,9 @@ static oems_status pack_fused(oems_pack* p, const std::vector<int>& part, bool* 
     // the rest, long x-runs and full tiles beat many short items
     const int share = std::max(1, std::min(sms, (int)std::lround(sms * (double)en->ncells_padded / cells)));
     bool ok = false;
-    OEMS_TRY(fused_pack_tune(en, share, &ok));
-    if (!ok) return OEMS_OK;
+    const oems_status st = fused_pack_tune(en, share, &ok);
+    if (!ok) give_back();
+    if (st != OEMS_OK || !ok) return st;
   }
   for (int i : part) {
     oems_engine* en = p->en[i];

@@ -332,3 +332,17 @@ def test_memory_that_is_tight_once_is_not_held_against_an_engine(child):
     e.run_batch(batch(4))
     assert fused(e)
     """)
+
+
+def test_a_pack_that_cannot_run_fused_holds_nothing_for_it(child):
+    child("""
+    knob("capacity", 1 << 30)
+    e = [engine((40, 41, 44)), engine((40, 41, 44), kernels="register"), engine((20010, 3, 3), (20000, 0, 0, 0, 0, 0))]
+    for other in e[1:]:  # kernels asked for by name; profiles that no CTA holds
+        e[0].reset()
+        used = F.fake_pool_used()
+        p = oe.Pack([e[0], other])
+        p.run_batch([batch(4)] * 2)
+        assert launched("k_fused") == 0 and launched("k_update_h_pack") > 0
+        assert F.fake_pool_used() - used < 1 << 20
+    """)

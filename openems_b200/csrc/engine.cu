@@ -27,6 +27,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <system_error>
 #include <thread>
@@ -685,6 +686,7 @@ struct oems_engine {
   // graphs keyed by span length and current buffers; invalidated when any
   // baked pointer changes
   std::map<int, cudaGraphExec_t> graphs;
+  std::set<int> seen;  // spans of fused passes launched without a graph so far
   uint64_t graph_epoch = 0, built_epoch = ~0ull;
 
   // per-kernel profiling
@@ -728,6 +730,7 @@ struct EngineScope {
 static void drop_graphs(oems_engine* en) {
   for (auto& kv : en->graphs) cudaGraphExecDestroy(kv.second);
   en->graphs.clear();
+  en->seen.clear();
 }
 
 static Geom make_geom(const oems_engine* en, int block, int ichunk) {
@@ -1498,6 +1501,7 @@ static oems_status launch_steps_profiled(oems_engine* en, int steps) {
 static std::mutex& tune_mutex();
 static oems_status launch_steps_fused(oems_engine* en, int steps);
 static uint64_t fused_launches(const oems_engine* en, int steps);
+static int fused_piece(const oems_engine* en, int steps);
 static void fused_swap(oems_engine* en);
 static void fused_rewind(oems_engine* en, int parity) {
   if (en->fus.parity != parity) fused_swap(en);
@@ -1546,8 +1550,24 @@ static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
   return OEMS_OK;
 }
 
+// Whether a span of fused passes is better launched pass by pass: a graph costs
+// 10 us a launch to make (a new 144^3 engine with dispersive media spent 34 ms
+// on one of 400 steps, whose run takes 39) and its replay saves next to nothing
+// where a pass takes longer than its launch.  So the first run of a length goes
+// without, and the next makes the graph.
+static bool first_of_length(oems_engine* en, int steps) {
+  if (en->built_epoch != en->graph_epoch) {
+    drop_graphs(en);
+    en->built_epoch = en->graph_epoch;
+  }
+  const int key = 2 * steps + en->fus.parity;
+  if (en->graphs.count(key)) return false;
+  if (en->seen.size() >= 4 * kMaxGraphs) en->seen.clear();
+  return en->seen.insert(key).second;
+}
+
 // Runs batch steps [base, base + steps).
-static oems_status run_span(oems_engine* en, long long base, int steps) {
+static oems_status run_piece(oems_engine* en, long long base, int steps) {
   if (need_post(en) || en->tfsf.on) {
     k_set_i64<<<1, 1, 0, en->stream>>>(en->d_base.p, base);
     OEMS_CUDA(cudaGetLastError());
@@ -1558,6 +1578,8 @@ static oems_status run_span(oems_engine* en, long long base, int steps) {
       en->prof_ev.resize(256, nullptr);
       for (auto& e : en->prof_ev) OEMS_CUDA(cudaEventCreate(&e));
     }
+    OEMS_TRY(launch_steps_fused(en, steps));
+  } else if (en->fus.use && first_of_length(en, steps)) {
     OEMS_TRY(launch_steps_fused(en, steps));
   } else if (en->profiling) {
     OEMS_TRY(launch_steps_profiled(en, steps));
@@ -1572,6 +1594,15 @@ static oems_status run_span(oems_engine* en, long long base, int steps) {
     OEMS_CUDA(e);
   }
   en->last_launches += en->fus.use ? fused_launches(en, steps) : (uint64_t)steps * kernels_per_step(en);
+  return OEMS_OK;
+}
+
+// Runs batch steps [base, base + steps); long spans of fused passes in pieces
+// of one length, so that the graph that is made is small and is used in the
+// batch that made it.
+static oems_status run_span(oems_engine* en, long long base, int steps) {
+  const int piece = en->fus.use ? fused_piece(en, steps) : steps;
+  for (int s = 0; s < steps; s += piece) OEMS_TRY(run_piece(en, base + s, std::min(piece, steps - s)));
   return OEMS_OK;
 }
 

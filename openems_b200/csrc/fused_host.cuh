@@ -845,13 +845,29 @@ static oems_status launch_steps_fused(oems_engine* en, int steps) {
   return OEMS_OK;
 }
 
+// Launches of a pass and what follows it.
+static int fused_pass_launches(const oems_engine* en) {
+  const FusedPlan& p = en->fus.current(fused_max_steps(en));
+  const int per = (p.items[0] ? 1 : 0) + (p.items[1] ? 1 : 0);
+  if (fused_hooks(en)) return per + ext_kernels(en) + post_kernels(en);
+  return per + (int)(en->fdumps.size() + en->boxes.size());
+}
+
 static uint64_t fused_launches(const oems_engine* en, int steps) {
   const int most = fused_max_steps(en);
   const uint64_t passes = (uint64_t)(steps + most - 1) / most;
-  const FusedPlan& p = en->fus.current(most);
-  const uint64_t fd = en->fdumps.size() + en->boxes.size(), per = (p.items[0] ? 1 : 0) + (p.items[1] ? 1 : 0);
-  if (fused_hooks(en)) return passes * (per + ext_kernels(en) + post_kernels(en));
-  return passes * (per + fd) + (en->nprobe() > 0 ? 1 : 0);
+  return passes * fused_pass_launches(en) + (!fused_hooks(en) && en->nprobe() > 0 ? 1 : 0);
+}
+
+// Steps of the pieces a span is run in: as even as it divides, of at most 256
+// launches (2.6 ms to make a graph of, under 1% of a piece between two of them),
+// and of four steps' multiples, which come back to the same buffers.
+constexpr int kGraphLaunches = 256;
+static int fused_piece(const oems_engine* en, int steps) {
+  const int most = std::max(4, kGraphLaunches / std::max(1, fused_pass_launches(en)) * fused_max_steps(en) / 4 * 4);
+  if (steps <= most) return steps;
+  const int pieces = (steps + most - 1) / most;
+  return ((steps + pieces - 1) / pieces + 3) / 4 * 4;
 }
 
 }  // namespace oems

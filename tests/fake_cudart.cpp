@@ -48,7 +48,7 @@ std::map<void*, Block>& blocks() {
   static std::map<void*, Block> m;
   return m;
 }
-long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, instantiated = 0;
+long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, instantiated = 0, captured = 0, largest = 0;
 thread_local cudaError_t last = cudaSuccess;
 thread_local int capturing = 0;
 
@@ -103,6 +103,7 @@ cudaError_t launch(const void* f) {
   if (refuse("fail_kernel", "pass_kernel")) return ret(cudaErrorLaunchOutOfResources);
   std::lock_guard<std::recursive_mutex> lk(mu);
   launched()[names().count(f) ? names()[f] : "?"]++;
+  if (capturing) largest = std::max(largest, ++captured);
   return cudaSuccess;
 }
 CUresult encode(...) { return CUDA_SUCCESS; }
@@ -128,6 +129,7 @@ long long fake_pool_used() { return pooled; }
 long long fake_pinned() { return pinned; }  // bytes now
 long long fake_pins() { return pins; }      // calls so far
 long long fake_instantiated() { return instantiated; }
+long long fake_largest_graph() { return largest; }  // kernels in it
 
 cudaError_t cudaMalloc(void** p, size_t n) { return alloc(p, n, false); }
 cudaError_t cudaFree(void* p) { return give(p); }
@@ -263,6 +265,7 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
 
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
   ++capturing;
+  captured = 0;
   return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {

@@ -22,7 +22,7 @@ import openems_b200._native as N
 N.LIB_PATH = %r
 import openems_b200 as oe
 L, F = N.lib(), ctypes.CDLL(N.LIB_PATH)
-for f in ("fake_launched", "fake_pool_used", "fake_pinned", "fake_pins", "fake_instantiated"):
+for f in ("fake_launched", "fake_pool_used", "fake_pinned", "fake_pins", "fake_instantiated", "fake_largest_graph"):
     getattr(F, f).restype = ctypes.c_longlong
 F.fake_set.argtypes = [ctypes.c_char_p, ctypes.c_longlong]
 
@@ -154,27 +154,24 @@ def test_no_room_for_taps_shortens_the_spans(child):
     """)
 
 
-# of the three kernel launches (two passes of 3 steps, the first swaps the
-# buffers), the second fails; the graph cannot be made; it cannot be launched
-@pytest.mark.parametrize("knobs", ['knob("pass_kernel", 1), knob("fail_kernel", 1)', 'knob("fail_instantiate", 1)',
-                                   'knob("fail_graph_launch", 1)'])
-@pytest.mark.parametrize("layers,again", [(None, False), ((4,) * 6, True)])
-def test_a_graph_that_fails_leaves_the_fields_current(child, knobs, layers, again):
+# A span's first run goes without a graph, per parity of the buffers.  The
+# second of two captured passes (which swap the buffers) cannot be launched; the
+# graph cannot be made; it cannot be launched, when new or when kept.
+@pytest.mark.parametrize("steps,runs,knobs", [(3, 1, 'knob("pass_kernel", 1), knob("fail_kernel", 1)'),
+                                              (1, 2, 'knob("fail_instantiate", 1)'), (1, 2, 'knob("fail_graph_launch", 1)'),
+                                              (1, 4, 'knob("fail_graph_launch", 1)')])
+@pytest.mark.parametrize("layers", [None, (4,) * 6])
+def test_a_graph_that_fails_leaves_the_fields_current(child, steps, runs, knobs, layers):
     """(Kernels do nothing here: what was written must come back.)"""
     child(f"""
     e = engine((20, 21, 22), {layers}, autotune=False)
-    e.run_batch(batch(2))  # (tables and buffers are there)
-    steps = 1 if "kernel" not in {knobs!r} else 3
-    if {again}:  # a graph kept from before, launched again
-        for _ in range(2):
-            e.run_batch(batch(steps))
-            e.run_batch(batch(steps + 4))
-        steps = steps if "launch" in {knobs!r} else steps + 8
+    for _ in range({runs}):
+        e.run_batch(batch({steps}))
     f = np.random.default_rng(0).standard_normal((2, 3, 20, 21, 22), dtype=np.float32)
     e.write_fields(f[0], f[1])
     {knobs}
     try:
-        e.run_batch(batch(steps))
+        e.run_batch(batch({steps}))
     except N.CudaError:
         pass
     else:
@@ -190,10 +187,11 @@ def test_graphs_of_both_parities_are_kept(child):
     child("""
     e = engine((20, 21, 22), autotune=False)
     lengths = (1, 3, 5, 9, 11, 13, 17, 19)
-    for _ in range(2):
+    for _ in range(5):
         for n in lengths:
             e.run_batch(batch(n))
     before = F.fake_instantiated()
+    assert before > 0
     for _ in range(3):
         for n in lengths:
             e.run_batch(batch(n))
@@ -345,4 +343,38 @@ def test_a_pack_that_cannot_run_fused_holds_nothing_for_it(child):
         p.run_batch([batch(4)] * 2)
         assert launched("k_fused") == 0 and launched("k_update_h_pack") > 0
         assert F.fake_pool_used() - used < 1 << 20
+    """)
+
+
+def test_graphs_of_long_spans_are_small(child):
+    """An engine's first batch of 400 steps with hooks and a recorder: no graph
+    of thousands of launches, and none for what is run once."""
+    child("""
+    e = engine((30, 31, 32), (4,) * 6, autotune=False)
+    e.add_dispersive(oe.DrudeMaterial(2e11, 1e9), np.array([[8, 8, 8]], dtype=np.uint64))
+    oe.fdtd.Nf2ffBox(e, (6, 6, 6), (20, 20, 20), [1e9])
+    assert e.run_batch(batch(400)).timesteps_executed == 400
+    assert 0 < F.fake_largest_graph() <= 256 and F.fake_instantiated() <= 2
+    for _ in range(3):
+        e.run_batch(batch(400))
+    assert F.fake_instantiated() <= 4
+    plain, before = engine((30, 31, 32), autotune=False), F.fake_instantiated()
+    plain.run_batch(batch(100))
+    assert F.fake_instantiated() == before
+    plain.run_batch(batch(100)), plain.run_batch(batch(100))
+    assert F.fake_instantiated() == before + 1
+    """)
+
+
+def test_pieces_of_a_span_are_all_run(child):
+    """Every step of spans around the pieces' lengths, probes included."""
+    child("""
+    e = engine((20, 21, 22), (4,) * 6, autotune=False, graphs=False)
+    e.add_point_probe(0, (3, 3, 3))
+    e.run_batch(batch(1))
+    for n in (511, 512, 513, 700, 1023, 1025, 3003):  # (one launch a pass: 512 steps a piece)
+        launched("", True)
+        e.run_batch(batch(n))
+        passes, sums = launched("k_fused"), launched("k_probe_sums")
+        assert passes == (n + 1) // 2 and sums == launched("k_set_i64") == -(-n // 512), (n, passes, sums)
     """)

@@ -26,7 +26,7 @@ NVCC_FLAGS = [
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-O2,-fvisibility=hidden",
     "--expt-relaxed-constexpr",
-    "-shared", "--split-compile=0",
+    "-shared", "--threads=0",
 ]
 
 

@@ -129,3 +129,11 @@ def test_interface_entry_points_refuse_null_arguments():
         == N.ERR_INVALID_ARGUMENT
     assert L.oems_engine_eval_terms(None, None, 0, 0, ctypes.byref(out)) == N.ERR_INVALID_ARGUMENT
     assert L.oems_engine_set_cells(None, 0, None, None, 1, 0) == N.ERR_INVALID_ARGUMENT
+
+
+def test_the_build_does_not_depend_on_the_machine():
+    """Split compilation shares a module's functions out as threads come free:
+    builds of one source differed (356 or 64 bytes of spills in the two-step
+    pass over CPML slabs), and with them speed by up to 12%."""
+    from openems_b200 import build
+    assert not any("split-compile" in f for f in build.NVCC_FLAGS)

@@ -2160,7 +2160,10 @@ static oems_status run_batch(oems_engine* en, const oems_batch* b, oems_batch_re
   en->last_launches = 0;
   bool fused = false;
   OEMS_TRY(fused_ready(en, &fused));
-  if (fused && en->fus.tuned != fused_max_steps(en)) OEMS_TRY(fused_tune(en, &fused));
+  if (fused && en->fus.tuned != fused_max_steps(en)) {
+    OEMS_TRY(fused_tune(en, &fused));
+    if (fused) OEMS_TRY(fused_or_separate(en, &fused));
+  }
   if (fused != en->fus.use || en->fus.packed) en->graph_epoch++;
   en->fus.use = fused;
   en->fus.packed = false;

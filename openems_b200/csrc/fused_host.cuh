@@ -535,7 +535,8 @@ static void launch_pass(FusedKernel k, const FusedArgs& a, int grid, int nt, siz
 // One pass of p.steps steps, starting at step `local` of the span: the boxes
 // with slabs on a second stream beside the others (they read and write the
 // same buffers, but no cell is written by both).
-static cudaError_t launch_fused(oems_engine* en, const FusedPlan& p, int local, bool posts) {
+// early: the launch may start while the kernel before it drains.
+static cudaError_t launch_fused(oems_engine* en, const FusedPlan& p, int local, bool posts, bool early = true) {
   FusedArgs a = fused_args(en, local, posts);
   const bool fork = p.items[0] && p.items[1] && side_stream(en);
   cudaStream_t side = fork ? en->side : en->stream;
@@ -547,12 +548,12 @@ static cudaError_t launch_fused(oems_engine* en, const FusedPlan& p, int local, 
     a.nbox = p.ncpml;
     std::copy(p.box, p.box + p.ncpml, a.box);
     a.pairs = p.pairs;
-    launch_pass(pick_fused(en, p.steps, true), a, p.items[1], p.nt[1], p.smem[1], side, !fork);
+    launch_pass(pick_fused(en, p.steps, true), a, p.items[1], p.nt[1], p.smem[1], side, early && !fork);
   }
   if (p.items[0]) {
     a.nbox = p.nbox - p.ncpml;
     std::copy(p.box + p.ncpml, p.box + p.nbox, a.box);
-    launch_pass(pick_fused(en, p.steps, false), a, p.items[0], p.nt[0], p.smem[0], en->stream, !p.items[1]);
+    launch_pass(pick_fused(en, p.steps, false), a, p.items[0], p.nt[0], p.smem[0], en->stream, early && !p.items[1]);
   }
   if (fork) {
     cudaEventRecord(en->join_ev, side);
@@ -621,13 +622,15 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
     const size_t most = cached || !time_it ? 1 : steps != longest ? 3 : small ? 30 : 12;
     if (c.size() > most) c.resize(most);
     FusedPlan best = c[0];
-    if (c.size() > 1) {
+    if (c.size() > 1 || (steps == longest && time_it && !cached)) {
       float best_ms = 1e30f;
       for (FusedPlan& p : c) {
-        OEMS_CUDA(launch_fused(en, p, 0, false));
-        const int kReps = small ? 8 : 3;
+        // (a one-step pass has a hook or a recorder before it, not another pass)
+        const bool early = longest > 1;
+        OEMS_CUDA(launch_fused(en, p, 0, false, early));
+        const int kReps = (int)std::max<long long>(3, std::min<long long>(8, 24000000 / en->ncells_padded));
         OEMS_CUDA(cudaEventRecord(en->ev0, en->stream));
-        for (int r = 0; r < kReps; ++r) OEMS_CUDA(launch_fused(en, p, 0, false));
+        for (int r = 0; r < kReps; ++r) OEMS_CUDA(launch_fused(en, p, 0, false, early));
         OEMS_CUDA(cudaEventRecord(en->ev1, en->stream));
         OEMS_CUDA(cudaEventSynchronize(en->ev1));
         float ms = 0.f;
@@ -655,6 +658,48 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
   F.tuned = longest;
   *ok = true;
   en->graph_epoch++;
+  return OEMS_OK;
+}
+
+// Milliseconds a step of the fastest candidate of a tuning report: passes of
+// `steps` (fused: true), or the separate kernels.
+static float best_of_report(const std::vector<oems_tune_entry>& report, bool fused, int steps) {
+  float best = 1e30f;
+  for (const oems_tune_entry& t : report)
+    if ((t.kind == 5) == fused && (!fused || t.extra % 10 == steps)) best = std::min(best, t.ms / (float)t.reps);
+  return best;
+}
+
+// Whether the tuned passes are to be taken, by the times of the two.  Two-step
+// passes were the faster ones on every grid measured (1.02 to 3 times, 24^3 to
+// 256^3, both coefficient forms) but a single plane's, which has nothing to
+// march through (1 x 1500 x 1500: 30.5 us a step, separate 21.4).  One-step
+// passes lose to kernels that find their arrays in the L2: 24^3 to 64^3 with
+// CPML and dispersive cells 22 to 25 us a step, separate 17.5 to 21; 121 x 196 x
+// 123, compressed, 81 against 70 there and 49.5 against 43.5 with Mur faces; but
+// 95 against 172 at 200^3 with Mur faces.  So where one of these holds the
+// separate kernels are tuned too, and taken if they are faster.  kHookUs: what
+// the hooks around a pass cost more than around the pair (their launches do not
+// hide behind its second kernel): 1.5 to 5 us measured, with one to four hooks.
+// The pair is not timed where its bytes alone, past the L2, take longer.
+constexpr float kHookUs = 3.0f;
+constexpr double kL2Bytes = 126e6, kPeakBytes = 6.5e9;  // per ms: the measured copy rate
+static oems_status fused_or_separate(oems_engine* en, bool* yes) {
+  FusedHost& F = en->fus;
+  const int longest = fused_max_steps(en);
+  if ((en->flags & OEMS_ENGINE_NO_AUTOTUNE) || (longest > 1 && en->nx > 1)) return OEMS_OK;
+  const std::vector<oems_tune_entry> passes = en->tune_report;
+  const float pass = best_of_report(passes, true, longest) + (fused_hooks(en) ? kHookUs * 1e-3f : 0.0f);
+  const double cells = (double)en->nx * en->ny * en->nz, coefs = en->id_bytes ? en->id_bytes : 24;
+  const double held = cells * (6 * en->elem + (en->id_bytes ? en->id_bytes : 48));
+  if (held > 2 * kL2Bytes && pass < 2 * cells * (9 * en->elem + coefs) / kPeakBytes) return OEMS_OK;
+  if (!en->tuned) OEMS_TRY(autotune(en));
+  *yes = !(best_of_report(en->tune_report, false, 0) < pass);
+  en->tune_report.insert(en->tune_report.begin(), passes.begin(), passes.end());
+  if (!*yes) {
+    F.state = -1;
+    fused_release(en);
+  }
   return OEMS_OK;
 }
 

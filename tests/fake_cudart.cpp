@@ -29,6 +29,8 @@ std::map<std::string, long long>& knobs() {
       {"fail_graph_launch", 0}, // graph launches to refuse
       {"fail_kernel", 0},       // kernel launches to refuse ...
       {"pass_kernel", 0},       // ... after letting this many through
+      {"pass_ns", 10000},       // time of a fused pass' launch between two events
+      {"update_ns", 10000},     // ... of an update kernel's
   };
   return k;
 }
@@ -49,6 +51,7 @@ std::map<void*, Block>& blocks() {
   return m;
 }
 long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, instantiated = 0, captured = 0, largest = 0;
+long long clock_ns = 0;  // of the launches so far
 thread_local cudaError_t last = cudaSuccess;
 thread_local int capturing = 0;
 
@@ -102,7 +105,10 @@ cudaError_t give(void* p) {
 cudaError_t launch(const void* f) {
   if (refuse("fail_kernel", "pass_kernel")) return ret(cudaErrorLaunchOutOfResources);
   std::lock_guard<std::recursive_mutex> lk(mu);
-  launched()[names().count(f) ? names()[f] : "?"]++;
+  const std::string name = names().count(f) ? names()[f] : "?";
+  launched()[name]++;
+  if (name.find("k_fused") != std::string::npos) clock_ns += knobs()["pass_ns"];
+  if (name.find("k_update") != std::string::npos) clock_ns += knobs()["update_ns"];
   if (capturing) largest = std::max(largest, ++captured);
   return cudaSuccess;
 }
@@ -251,15 +257,22 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
-  *e = reinterpret_cast<cudaEvent_t>(8);
+  *e = reinterpret_cast<cudaEvent_t>(new long long(0));
   return cudaSuccess;
 }
 cudaError_t cudaEventCreate(cudaEvent_t* e) { return cudaEventCreateWithFlags(e, 0); }
-cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) {
+  delete reinterpret_cast<long long*>(e);
+  return cudaSuccess;
+}
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  *reinterpret_cast<long long*>(e) = clock_ns;
+  return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
-  *ms = 1.0f;
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) {
+  *ms = (float)(*reinterpret_cast<long long*>(b) - *reinterpret_cast<long long*>(a)) * 1e-6f;
   return cudaSuccess;
 }
 

@@ -303,7 +303,7 @@ def test_plans_of_one_step_engines_are_searched(child):
     child("""
     def tried(e):
         e.run_batch(batch(4))
-        return sorted(r["extra"] % 10 for r in e.tune_report())
+        return sorted(r["extra"] % 10 for r in e.tune_report() if r["kind"] == 5)
     plain = engine((30, 31, 32))
     assert tried(plain).count(2) > 10 and launched("k_fused") > 0
     mur = engine((30, 31, 32))
@@ -377,4 +377,33 @@ def test_pieces_of_a_span_are_all_run(child):
         e.run_batch(batch(n))
         passes, sums = launched("k_fused"), launched("k_probe_sums")
         assert passes == (n + 1) // 2 and sums == launched("k_set_i64") == -(-n // 512), (n, passes, sums)
+    """)
+
+
+# us of a pass' launch and of an update kernel's; the update takes two a step
+@pytest.mark.parametrize("what,dims,pass_us,update_us,want", [
+    ("mur", (30, 31, 32), 20, 13, True), ("mur", (30, 31, 32), 20, 11, False),
+    ("recorder", (30, 31, 32), 20, 10.1, True), ("recorder", (30, 31, 32), 20, 9.9, False),
+    ("plain", (30, 31, 32), 80, 10, True), ("plain", (1, 80, 90), 80, 21, True), ("plain", (1, 80, 90), 80, 19, False),
+    ("mur", (170, 171, 172), 80, 1, True)])
+def test_one_step_passes_are_taken_where_they_are_faster(child, what, dims, pass_us, update_us, want):
+    """Timed against the separate kernels, but for a grid past the L2 whose
+    bytes alone take those longer (5 M cells: 92 us)."""
+    child(f"""
+    knob("pass_ns", int({pass_us} * 1000)), knob("update_ns", int({update_us} * 1000))
+    def make():
+        e = engine({dims})
+        if {what!r} == "mur":
+            e.add_mur(oe.MurAbcConfig.all(1))
+        if {what!r} == "recorder":
+            oe.fdtd.Nf2ffBox(e, (4, 4, 4), (15, 15, 15), [1e9])
+        return e
+    for e in (make(), make()):  # tuned, and from what was tuned
+        for _ in range(2):
+            e.run_batch(batch(6))
+            assert fused(e) == {want}, e.tune_report()
+        used = F.fake_pool_used()
+    e = engine({dims}, autotune=False)
+    e.run_batch(batch(6))
+    assert fused(e)
     """)

@@ -6,15 +6,17 @@ import pytest
 import oracle
 import openems_b200 as oe
 from scenarios import dispersive_scenarios, run_engine, run_oracle, upml_scenarios
-from test_gpu_parity import KERNELS, assert_parity
+from test_gpu_parity import KERNELS, ROUTES, assert_parity, route
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kernels", KERNELS)
+@pytest.mark.parametrize("kernels", ROUTES)
 @pytest.mark.parametrize("sc", dispersive_scenarios(), ids=lambda s: s.name)
 def test_extension_scenarios(sc, kernels):
-    assert_parity(run_engine(sc, kernels=kernels), run_oracle(sc))
+    got = run_engine(sc, **route(kernels))
+    assert (got["engine"].launch_info()["staged"] == 5) == (kernels == "fused")
+    assert_parity(got, run_oracle(sc))
 
 
 @pytest.mark.parametrize("kernels", KERNELS)
@@ -90,7 +92,7 @@ def _port_run(kernels):
     op.set_pec((12, 13, 12, 13, 9, 15))
     op.set_pec((12, 13, 12, 13, 16, 22))
     port = oe.LumpedPort(1, 50.0, pos, d, excite=1.0).apply(op)
-    eng = oe.Engine(op, kernels=kernels)
+    eng = oe.Engine(op, **route(kernels))
     eng.add_cpml(oe.CpmlBoundaries.uniform(6))
     port.add_probes(eng, freqs)
     wave = oe.Excitation.gaussian_modulated(8e9, 0.75, d, pos)
@@ -122,7 +124,7 @@ def _port_run(kernels):
     return eng, port, s, (du, di), freqs
 
 
-@pytest.mark.parametrize("kernels", KERNELS)
+@pytest.mark.parametrize("kernels", ROUTES)
 def test_lumped_port_s11(kernels):
     eng, port, s, (du, di), freqs = _port_run(kernels)
     port.calc_port(eng)

@@ -7,7 +7,7 @@ import oracle
 from oracle import nf2ff_ref as R
 import openems_b200 as oe
 from scenarios import make_operator, Scenario
-from test_gpu_parity import KERNELS
+from test_gpu_parity import ROUTES, route
 
 pytestmark = pytest.mark.gpu
 
@@ -32,7 +32,7 @@ BOX = ((5, 4, 6), (17, 15, 21), [6e9, 9e9], (1, 1, 0, 1, 1, 1), 1)
 def run_both(kernels):
     sc = fd_scenario()
     op = make_operator(sc)
-    eng = oe.Engine(op, kernels=kernels)
+    eng = oe.Engine(op, **route(kernels))
     eng.add_cpml(sc.cpml)
     ids = [eng.add_field_dft(r, f, m, ss, iv) for r, f, m, ss, iv in DUMPS]
     lo, hi, bf, dirs, biv = BOX
@@ -58,9 +58,10 @@ def run_both(kernels):
     return eng, ids, box, s, oids, obox, [np.asarray(v, dtype=np.float64) for v in lines]
 
 
-@pytest.mark.parametrize("kernels", KERNELS)
+@pytest.mark.parametrize("kernels", ROUTES)
 def test_field_dft_and_box_bit_exact(kernels):
     eng, ids, box, s, oids, obox, _ = run_both(kernels)
+    assert (eng.launch_info()["staged"] == 5) == (kernels == "fused")
     e, h = eng.read_fields()
     assert np.array_equal(np.concatenate([e, h]), s.fields())
     for (r, f, m, ss, iv), d, od in zip(DUMPS, ids, oids):

@@ -141,3 +141,42 @@ def test_against_the_oracle(sc):
     got = run_engine(sc)
     assert got["engine"].launch_info()["staged"] == 5
     assert_parity(got, run_oracle(sc))
+
+
+@pytest.mark.parametrize("layers,mur,disp,storage", [((8, 0, 6, 10, 0, 9), 0, False, "f32"), (None, 0, False, "f16"),
+                                                     ((6,) * 6, 0, True, "f32"), (None, 2, False, "f32")])
+def test_state_after_an_odd_number_of_passes(layers, mur, disp, storage):
+    """The buffers a pass swaps are the current ones for whatever reads or
+    writes the state next: energies, checkpoints to and from the separate
+    kernels, resets and written fields."""
+    sc = random_scenario(13, (30, 31, 35), layers, mur, disp)  # 25 + 12 steps: 19 passes, or 37
+
+    def more(run, n, start):
+        eng, dt = run["engine"], run["operator"].timestep()
+        eng.run_batch(oe.EngineBatch(num_steps=n, excitations=[
+            oe.ScheduledExcitation.from_excitation(x, start, n, dt) for x in sc.excitations]))
+        return np.concatenate(eng.read_fields())
+
+    def fresh(**kw):
+        return run_engine(sc, storage=storage, autotune=False, **kw)
+
+    def story(run, other):
+        eng, out = run["engine"], []
+        out += [run["fields"], np.array(eng.energy())]
+        blob = eng.save_state()
+        out += [more(run, 9, 37), more(run, 3, 46)]  # 5 passes more, then 2
+        eng.load_state(blob)
+        out += [np.concatenate(eng.read_fields()), np.array(eng.energy()), more(run, 9, 37)]
+        other["engine"].load_state(blob)
+        out += [more(other, 9, 37)]
+        f = np.random.default_rng(1).standard_normal((2, 3, 30, 31, 35)).astype(np.float16).astype(np.float32)
+        eng.write_fields(f[0], f[1] / 512)
+        out += [np.concatenate(eng.read_fields()), more(run, 5, 46)]
+        eng.reset()
+        out += [np.concatenate(eng.read_fields()), more(run, 25, 0), np.array(eng.energy())]
+        return out
+
+    a, b = fresh(), fresh(kernels="register")
+    assert a["engine"].launch_info()["staged"] == 5 and b["engine"].launch_info()["staged"] != 5
+    for x, y in zip(story(a, fresh(kernels="register")), story(b, fresh())):
+        assert np.array_equal(x, y)

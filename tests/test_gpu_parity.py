@@ -61,6 +61,12 @@ def test_config1_64_pec_2000_steps(kernels):
 
 
 KERNELS = ("register", "staged", "split", "zsplit", "pipe")
+# ... and the fused passes (untimed, so that the tuner takes no other)
+ROUTES = KERNELS + ("fused",)
+
+
+def route(kernels):
+    return dict(autotune=False) if kernels == "fused" else dict(kernels=kernels)
 
 
 @pytest.mark.parametrize("kernels", KERNELS)

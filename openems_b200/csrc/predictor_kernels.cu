@@ -634,9 +634,15 @@ oems_status oems_pk_relu_bwd(float* dy, const float* y, int64_t n, void* stream)
 }
 
 oems_status oems_pk_colsum(const float* dy, int64_t rows, int w, float* db, void* stream) {
+  // The parts (two launches, 10 us and more) against a block per column: they
+  // pay from 12,288 rows of 33 to 128 columns on (10.3 us both; 4,096 x 128 9.6
+  // against 6.2, 65,536 x 128 12.3 against 36.9), 6,144 of 192 and 256 (10.3),
+  // 4,096 of 512 and 640 (11.4 against 12.3, 13.3 against 14.7) and 24,576 of 16
+  // (10.3); at 2,048 x 640 13.3 against 10.3.
+  const bool long_columns = rows >= (w < 32 ? 24576 : 4096) && rows * std::max(w, 128) >= 1570000;
   const int parts = 148;
   Workspace ws(stream);
-  if (rows >= 4096 && ws.get((size_t)parts * w * sizeof(float))) {
+  if (long_columns && ws.get((size_t)parts * w * sizeof(float))) {
     const long long per = (rows + parts - 1) / parts;
     float* part = static_cast<float*>(ws.p);
     if (w % 4 == 0 && aligned16(dy, dy))

@@ -61,7 +61,8 @@ def test_causal_columns(C, pad):
     assert np.allclose(dx.cpu().numpy(), ref, rtol=1e-6, atol=1e-6)
 
 
-@pytest.mark.parametrize("rows,w", [(4095, 33), (4096, 33), (5000, 128), (70001, 8)])
+@pytest.mark.parametrize("rows,w", [(4095, 33), (4096, 33), (5000, 128), (70001, 8), (12265, 128), (12266, 128), (4096, 640),
+                                    (24576, 3), (13001, 35)])
 def test_column_sums_and_relu(rows, w):
     x = rnd(rows, w)
     db = torch.empty(w, device="cuda")

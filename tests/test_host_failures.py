@@ -206,7 +206,7 @@ def test_no_workspace_takes_the_forms_without(child):
     def calls():
         a, b, c = (np.zeros(n, np.float32) for n in (128 * 4096, 640 * 4096, 128 * 640))
         N.check(L.oems_tc_gemm_bf16(a.ctypes.data, 4096, b.ctypes.data, 4096, c.ctypes.data, 640, 128, 640, 4096, 0.0, None, None))
-        N.check(L.oems_pk_colsum(a.ctypes.data, 4096, 128, c.ctypes.data, None))
+        N.check(L.oems_pk_colsum(b.ctypes.data, 20480, 128, c.ctypes.data, None))
         return [launched(k) for k in ("k_gemm_tc", "k_gemm_sum", "k_colsum_part", "k_colsumEPK")]
     assert calls() == [1, 1, 1, 0]
     knob("fail_pool_from", 0)
@@ -406,4 +406,17 @@ def test_one_step_passes_are_taken_where_they_are_faster(child, what, dims, pass
     e = engine({dims}, autotune=False)
     e.run_batch(batch(6))
     assert fused(e)
+    """)
+
+
+@pytest.mark.parametrize("rows,w,parts", [(4096, 33, False), (8192, 128, False), (12265, 128, False), (12266, 128, True),
+                                          (6132, 256, False), (6133, 256, True), (4095, 640, False), (4096, 640, True),
+                                          (2048, 640, False), (16384, 16, False), (24576, 16, True), (65536, 128, True)])
+def test_column_sums_in_parts_where_they_pay(child, rows, w, parts):
+    """From 4,096 rows on whatever the width, 8,192 x 128 took 10.2 us instead
+    of 8.2."""
+    child(f"""
+    x, y = np.zeros({rows} * {w}, np.float32), np.zeros({w}, np.float32)
+    N.check(L.oems_pk_colsum(x.ctypes.data, {rows}, {w}, y.ctypes.data, None))
+    assert (launched("k_colsum_part") == 1) == {parts} and (launched("k_colsumEPK") == 1) != {parts}
     """)

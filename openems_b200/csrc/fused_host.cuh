@@ -375,10 +375,14 @@ static double fused_cost(const FusedPlan& p, int sms, const int (&occ)[2], std::
   return *std::max_element(heap.begin(), heap.end());
 }
 
-// Grids below this many cells are tuned over more shapes: a pass takes tens
-// of microseconds, and latency the model does not see decides.  (One-step
-// passes, with fewer planes of lead-in, measure level with two-step ones there
-// when launched back to back, and a fifth slower inside a graph.)
+// Grids below this many cells are tuned over more shapes (30 instead of 12): a
+// pass takes tens of microseconds, and latency the model does not see decides.
+// 121 x 98 x 75 with CPML 25.7 -> 24.0 us a step, 48 x 160 x 70 20.4 -> 19.6, the
+// other twelve shapes below a million cells tried within 1%; the first batch
+// takes 3 to 14 ms more.  Above, 18 more shapes gave 1 to 3% (170^3 78.8 -> 76.5,
+// 256^3 188.9 -> 186.7, none at 200^3) for 20 to 30 ms.  (One-step passes, with
+// fewer planes of lead-in, measure level with two-step ones there when launched
+// back to back, and a fifth slower inside a graph.)
 constexpr long long kFusedSmall = 3000000;
 
 // Sets of the table a CTA's shared memory has room for: plans, and the tuning

@@ -477,12 +477,15 @@ oems_status oems_tc_gemm_bf16(const void* a, int lda, const void* b, int ldb, fl
   // few tiles and a long K (the weight gradients: 128 x 640 outputs over K =
   // 65,536 ran on 10 of 148 SMs, 215 us): the K range in parts of at least 8
   // blocks, as many as the SMs take in one wave.  Fewer than half the SMs
-  // busy, or the sum of the parts costs more than it gives.
+  // busy, or the sum of the parts costs more than it gives; so it does for
+  // outputs past 2^18 below K = 4,096 (640 x 640 and 1000 x 512 at 2,048: 17.4
+  // and 20.0 us in parts, 16.5 whole; level at 3,072; 20.6 against 24.7 and level
+  // at 4,096; 128 x 1024 at 2,048 14.4 against 16.5).
   const int nkb = (K + 63) / 64;
   p.splits = 1;
   p.kb_per = nkb;
   Workspace ws(stream);
-  if (tm * ((N + BN - 1) / BN) * 2 <= sms && nkb >= 32) {
+  if (tm * ((N + BN - 1) / BN) * 2 <= sms && nkb >= ((long long)M * N > (1 << 18) ? 64 : 32)) {
     long long fewest = -1;
     int split_bn = BN;
     for (int cand : {256, 128, 64}) {

@@ -44,10 +44,11 @@ def test_transpose(R, C, ldx, ldy):
     assert torch.equal(y[:, :R], x[:, :C].T) and not y[:, R:].any()
 
 
+@pytest.mark.parametrize("B,T", [(3, 37), (5, 9001)])  # the latter past the line of the 4-channel gather
 @pytest.mark.parametrize("C,pad", [(8, 0), (16, 8), (12, 4), (4, 3)])
-def test_causal_columns(C, pad):
+def test_causal_columns(C, pad, B, T):
     from oracle.tailnet_ref import col2im_causal, im2col_causal, round_bf16
-    B, T, ks, dil = 3, 37, 5, 4
+    ks, dil = 5, 4
     ldc = ks * C + pad
     x = rnd(B, T, C)
     cols = torch.zeros(B * T, ldc, dtype=torch.bfloat16, device="cuda")

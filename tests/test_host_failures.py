@@ -432,3 +432,14 @@ def test_gemm_split_where_it_pays(child, m, n, k, split):
     N.check(L.oems_tc_gemm_bf16(at[0], {k}, at[1], {k}, c.ctypes.data, {n}, {m}, {n}, {k}, 0.0, None, None))
     assert launched("k_gemm_tc") == 1 and (launched("k_gemm_sum") == 1) == {split}
     """)
+
+
+@pytest.mark.parametrize("b,t,c,wide", [(8, 64, 128, False), (1, 16, 8, False), (8, 128, 128, True), (4, 8192, 6, False)])
+def test_column_gather_form(child, b, t, c, wide):
+    """Small launches are shorter with the plain kernel (4.0 us against 4.2)."""
+    child(f"""
+    x, y = np.zeros({b} * {t} * {c} * 5 + 4, np.float32), np.zeros({b} * {t} * {c} + 4, np.float32)
+    at = [q.ctypes.data + -q.ctypes.data % 16 for q in (x, y)]
+    N.check(L.oems_pk_col2im_causal(at[0], 5 * {c}, at[1], {b}, {t}, {c}, 5, 2, None))
+    assert (launched("k_col2im_causal4") == 1) == {wide} and launched("k_col2im_causal") == 1
+    """)

@@ -358,16 +358,20 @@ OEMS_API oems_status oems_engine_reset(oems_engine* engine);
  * one field storage, with full coefficient arrays and only CPML, sources,
  * probes and probe DFTs attached.  oems_pack_run_batch runs batches[i] on
  * engine i for every i with batches[i] != NULL, with the results and state
- * oems_engine_run_batch would give each engine on its own (bit for bit),
- * but every half-step of all of them is one launch of the plain update
- * kernels over the grids without CPML and one of the CPML kernels over the
- * grids with it, replayed from CUDA graphs, with one post-step launch and
- * one energy launch pair for all.  The first batch times the update
- * kernels' CTA size, x-planes per work item and whether CPML grids enter
- * whole or split (below) on saved copies of the engines' state (restored
- * afterwards) and keeps the fastest; a batch whose engines hold under half
- * the cells of the tuned set tunes again.  oems_pack_set_shape fixes the
- * shape instead.  The batches must share num_steps,
+ * oems_engine_run_batch would give each engine on its own (bit for bit), by
+ * one of two routes.  Shared launches: every half-step of all engines is one
+ * launch of the plain update kernels over the grids without CPML and one of
+ * the CPML kernels over the grids with it, replayed from CUDA graphs, with
+ * one post-step launch and one energy launch pair for all; the first batch
+ * that runs them times the update kernels' CTA size, x-planes per work item
+ * and whether CPML grids enter whole or split (below) on saved copies of the
+ * engines' state (restored afterwards) and keeps the fastest, and a batch
+ * whose engines hold under half the cells of the tuned set tunes again.
+ * Fused passes: where every engine of the batch can take them, each engine's
+ * own passes on its own stream, side by side.  The first spans of a set of
+ * grids run by one, then by the other, on the clock, and the faster is kept
+ * for packs of such grids.  oems_pack_set_shape fixes the shape and with it
+ * the shared launches.  The batches must share num_steps,
  * sample_interval, check_interval and whether they carry an energy-decay end
  * condition, and their engines must be at the same timestep; each engine
  * keeps its own decay threshold, peak and termination step.  statuses[i] is
@@ -387,7 +391,9 @@ OEMS_API oems_status oems_pack_run_batch(oems_pack* pack, const oems_batch* cons
  * (plain kernels) and its slab cells (CPML kernels); 2 and 3 as 1 with the
  * CPML launch on a second stream beside the plain one (3: the plain
  * launch's grid cut by one CTA per SM to leave room for it).  Setting it
- * skips the tuning of the first batch. */
+ * keeps the pack on the shared launches and skips their tuning;
+ * oems_pack_shape reads the shape they have or would have (fused passes have
+ * shapes of their own: oems_engine_launch_info). */
 OEMS_API oems_status oems_pack_set_shape(oems_pack* pack, int32_t threads, int32_t ichunk,
                                          int32_t split);
 OEMS_API oems_status oems_pack_shape(const oems_pack* pack, int32_t* threads, int32_t* ichunk,

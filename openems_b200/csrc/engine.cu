@@ -1554,7 +1554,8 @@ static oems_status get_graph(oems_engine* en, int steps, cudaGraphExec_t* out) {
 // 10 us a launch to make (a new 144^3 engine with dispersive media spent 34 ms
 // on one of 400 steps, whose run takes 39) and its replay saves next to nothing
 // where a pass takes longer than its launch.  So the first run of a length goes
-// without, and the next makes the graph.
+// without, and the next makes the graph.  (Not in packs: passes launched one by
+// one for many engines keep the host busy and the engines apart.)
 static bool first_of_length(oems_engine* en, int steps) {
   if (en->built_epoch != en->graph_epoch) {
     drop_graphs(en);
@@ -1579,7 +1580,7 @@ static oems_status run_piece(oems_engine* en, long long base, int steps) {
       for (auto& e : en->prof_ev) OEMS_CUDA(cudaEventCreate(&e));
     }
     OEMS_TRY(launch_steps_fused(en, steps));
-  } else if (en->fus.use && first_of_length(en, steps)) {
+  } else if (en->fus.use && !en->fus.packed && first_of_length(en, steps)) {
     OEMS_TRY(launch_steps_fused(en, steps));
   } else if (en->profiling) {
     OEMS_TRY(launch_steps_profiled(en, steps));
@@ -4185,6 +4186,11 @@ struct oems_pack {
   bool tuned = false;
   bool shape_set = false;  // chosen by oems_pack_set_shape: never re-tuned
   double tuned_cells = 0;  // cells of the engines the shape was tuned on
+  // fused passes or shared launches, as decided for batches of these intervals
+  // and engines of this many cells (PackChoice)
+  int route = 0;
+  double route_cells = 0;
+  uint64_t route_si = 0, route_ci = 0;
 };
 
 namespace oems {
@@ -4585,6 +4591,41 @@ static bool pack_takes(const oems_engine* en) {
            !en->boxes.empty());
 }
 
+// Which of the two routes a set of engines takes: each engine's own fused
+// passes side by side, or the shared launches.  Neither is the faster one
+// throughout (us a step, fused / shared: 12 antennas of 1 M cells with CPML 340 /
+// 650; 30 of 64 x 60 x 70 with CPML 184 / 322, 8 of them 112 / 93; 100 of 20^3
+// sampled every 10 steps 167 / 84, 8 of 20^3 14 / 28): a graph and an energy
+// sample cost each engine their launches, and passes planned for a share of
+// the SMs fill them less well than launches over all grids.  Both give the same
+// bits, so the first spans of a set are run by one, then by the other, on the
+// clock, and the faster runs what follows.  Kept per process for sets of the
+// same grids.
+constexpr int kPackWarm[2] = {3, 2};  // spans before the clock (a graph is made of a length's first run, per parity)
+constexpr int kPackTimed = 4;         // spans on it ...
+constexpr uint64_t kPackSpan = 48;    // ... of at most this many steps
+struct PackKey {
+  int dev, storage;
+  uint64_t si, ci;
+  std::vector<std::array<int, 9>> en;  // sizes and slabs
+  bool operator<(const PackKey& o) const {
+    return std::tie(dev, storage, si, ci, en) < std::tie(o.dev, o.storage, o.si, o.ci, o.en);
+  }
+};
+struct PackChoice {
+  int route = 0;  // 0 being timed, 1 fused, 2 shared
+  int warm[2] = {0, 0}, spans[2] = {0, 0};
+  uint64_t steps[2] = {0, 0};
+  double sec[2] = {0, 0};
+  // shape of the shared launches, once tuned
+  bool tuned = false, split = false, fork = false;
+  int threads = 0, ichunk = 0, cut = 0;
+};
+static std::map<PackKey, PackChoice>& pack_choices() {
+  static std::map<PackKey, PackChoice> m;
+  return m;
+}
+
 static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches, oems_batch_result* results,
                                   oems_status* statuses) {
   const auto t_start = std::chrono::steady_clock::now();
@@ -4633,24 +4674,99 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
     OEMS_CUDA(cudaStreamSynchronize(en->stream));
   }
   DeviceGuard dg(p->device);
-  if (fused) {
-    p->active = part;
-    OEMS_TRY(pack_host_energy(p, part.size()));
-  } else {
-    OEMS_TRY(pack_layout(p, part));
-  }
-  // tuned on the first batch, and again when the engines in the batch hold
-  // under half the cells the shape was tuned on (a sweep's pack shrinks as
-  // its instances end)
   double cells = 0;
   for (int i : part) cells += (double)p->en[i]->nx * p->en[i]->ny * p->en[i]->nz;
-  if (!fused && !p->shape_set && (!p->tuned || cells < 0.5 * p->tuned_cells)) OEMS_TRY(pack_tune(p));
   const uint64_t si = b0->sample_interval, ci = b0->check_interval;
   const bool has_decay = b0->has_energy_decay_db != 0;
   const uint64_t t0 = R[part[0]].t0;
+  // the route: as decided before for this pack or for such a set, or on the clock
+  const bool may_fuse = fused;
+  PackKey key{p->device, p->storage, si, has_decay ? ci : 0, {}};
+  PackChoice choice;
+  if (may_fuse) {
+    for (int i : part) {
+      const oems_engine* en = p->en[i];
+      std::array<int, 9> k{en->nx, en->ny, en->nz};
+      if (en->cpml.on) std::copy(en->cpml.args.L, en->cpml.args.L + 6, k.begin() + 3);
+      key.en.push_back(k);
+    }
+    std::lock_guard<std::mutex> lock(tune_mutex());
+    auto hit = pack_choices().find(key);
+    if (hit != pack_choices().end()) choice = hit->second;
+    // (a pack shrinks as its engines end; half the cells left are another set)
+    if (choice.route == 0 && p->route && cells >= 0.5 * p->route_cells && p->route_si == key.si && p->route_ci == key.ci)
+      choice.route = p->route;
+  }
+  bool trial = may_fuse && choice.route == 0;
+  fused = may_fuse && (choice.route == 1 || (trial && choice.spans[0] < kPackTimed));
+  auto sync_route = [&]() -> oems_status {
+    if (fused)
+      for (int i : part) OEMS_CUDA(cudaStreamSynchronize(p->en[i]->stream));
+    else
+      OEMS_CUDA(cudaStreamSynchronize(p->stream));
+    return OEMS_OK;
+  };
+  // the shared launches over the engines still running; tuned on the first
+  // batch, and again when the engines hold under half the cells the shape was
+  // tuned on
+  auto to_shared = [&](const std::vector<int>& act) -> oems_status {
+    if (!p->shape_set && choice.tuned && !p->tuned) {
+      p->threads = choice.threads;
+      p->ichunk = choice.ichunk;
+      p->split = choice.split;
+      p->fork = choice.fork && p->side;
+      p->cut = choice.cut;
+      p->tuned = true;
+      p->tuned_cells = cells;
+      OEMS_TRY(pack_grids_any(p));
+    }
+    OEMS_TRY(pack_layout(p, act));
+    if (!p->shape_set && (!p->tuned || cells < 0.5 * p->tuned_cells)) OEMS_TRY(pack_tune(p));
+    choice.tuned = true;
+    choice.threads = p->threads;
+    choice.ichunk = p->ichunk;
+    choice.split = p->split;
+    choice.fork = p->fork;
+    choice.cut = p->cut;
+    return OEMS_OK;
+  };
+  p->active = part;
+  OEMS_TRY(pack_host_energy(p, part.size()));
+  if (!fused) OEMS_TRY(to_shared(part));
+  std::chrono::steady_clock::time_point clock0;
+  bool on_clock = false;
+  auto stop_clock = [&]() -> oems_status {
+    if (!on_clock) return OEMS_OK;
+    on_clock = false;
+    OEMS_TRY(sync_route());
+    choice.sec[fused ? 0 : 1] += std::chrono::duration<double>(std::chrono::steady_clock::now() - clock0).count();
+    return OEMS_OK;
+  };
   OEMS_CUDA(cudaEventRecord(p->ev0, p->stream));
   uint64_t s = 0;
   while (s < steps && !p->active.empty()) {
+    if (trial && choice.spans[fused ? 0 : 1] >= kPackTimed) {
+      OEMS_TRY(stop_clock());
+      if (fused) {
+        OEMS_TRY(sync_route());
+        fused = false;
+        const std::vector<int> act = p->active;
+        if (to_shared(act) != OEMS_OK) {
+          // (no room to tune them)
+          cudaGetLastError();
+          p->active = act;
+          p->tuned = false;
+          choice.route = 1;
+        }
+      } else {
+        choice.route = choice.sec[0] * (double)choice.steps[1] <= choice.sec[1] * (double)choice.steps[0] ? 1 : 2;
+      }
+      trial = choice.route == 0;
+      if (choice.route == 1) {
+        OEMS_TRY(sync_route());
+        fused = true;
+      }
+    }
     const uint64_t cur = t0 + s;
     uint64_t ev = UINT64_MAX;
     if (si > 0) ev = std::min(ev, (cur + si - 1) / si * si);
@@ -4662,6 +4778,21 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
     uint64_t span = steps - s;
     if (ev != UINT64_MAX && ev - cur + 1 < span) span = ev - cur + 1;
     span = std::min<uint64_t>(span, span_cap);
+    if (trial) {
+      const int k = fused ? 0 : 1;
+      span = std::min(span, kPackSpan);
+      if (choice.warm[k] < kPackWarm[k]) {
+        choice.warm[k]++;
+      } else {
+        if (!on_clock) {
+          OEMS_TRY(sync_route());
+          clock0 = std::chrono::steady_clock::now();
+          on_clock = true;
+        }
+        choice.spans[k]++;
+        choice.steps[k] += span;
+      }
+    }
     if (fused) {
       for (int i : p->active) {
         EngineScope guard(p->en[i]);
@@ -4722,8 +4853,20 @@ static oems_status pack_run_batch(oems_pack* p, const oems_batch* const* batches
     }
   }
   for (int i : p->active) R[i].executed = s;
+  OEMS_TRY(stop_clock());
+  if (may_fuse) {
+    std::lock_guard<std::mutex> lock(tune_mutex());
+    if (pack_choices().size() >= 256) pack_choices().clear();
+    pack_choices()[key] = choice;
+    if (choice.route) {
+      p->route = choice.route;
+      p->route_cells = cells;
+      p->route_si = key.si;
+      p->route_ci = key.ci;
+    }
+  }
   if (fused) {
-    for (int i : part) OEMS_CUDA(cudaStreamSynchronize(p->en[i]->stream));
+    OEMS_TRY(sync_route());
     p->active.clear();  // the shared launches' tables are not these engines'
   }
   // probe DFTs of each engine's executed steps

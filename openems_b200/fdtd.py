@@ -1404,14 +1404,18 @@ def _batch_result(r, samples, cap) -> "BatchResult":
 
 
 class Pack:
-    """Several engines stepped by shared launches (oems_pack_*): one launch
-    per half-step of the plain update kernels over the grids without CPML
-    and one of the CPML kernels over the grids with it, a post-step launch
-    with a CTA per engine and two energy launches for all.  Each engine ends
-    a batch with the bits oems_engine_run_batch would give it.  The first
-    batch tunes the launch shape (CTA size, x-planes per work item, CPML
-    grids whole or split into box and slabs) unless set_shape chose one.  The engines need full coefficients and only CPML,
-    sources, probes and probe DFTs; keep them alive while the pack exists."""
+    """Several engines stepped together (oems_pack_*): each engine's own fused
+    passes side by side, or shared launches (one per half-step of the plain
+    update kernels over the grids without CPML and one of the CPML kernels
+    over the grids with it, a post-step launch with a CTA per engine and two
+    energy launches for all), whichever is faster for such grids: the first
+    spans run by each in turn, on the clock.  Each engine ends a batch with
+    the bits oems_engine_run_batch would give it.  The first shared launches
+    are tuned (CTA size, x-planes per work item, CPML grids whole or split
+    into box and slabs) unless set_shape chose a shape, which also keeps the
+    pack on them.  The engines need full coefficients and only CPML, sources,
+    probes and probe DFTs, at every batch; keep them alive while the pack
+    exists."""
 
     def __init__(self, engines: Sequence["Engine"]):
         self.engines = list(engines)

@@ -9,12 +9,14 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 
 namespace {
 
@@ -31,6 +33,7 @@ std::map<std::string, long long>& knobs() {
       {"pass_kernel", 0},       // ... after letting this many through
       {"pass_ns", 10000},       // time of a fused pass' launch between two events
       {"update_ns", 10000},     // ... of an update kernel's
+      {"real_time", 0},         // 1: that time passes on the host
   };
   return k;
 }
@@ -54,6 +57,7 @@ long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 
 long long clock_ns = 0;  // of the launches so far
 thread_local cudaError_t last = cudaSuccess;
 thread_local int capturing = 0;
+thread_local long long captured_ns = 0;
 
 cudaError_t ret(cudaError_t e) {
   if (e != cudaSuccess) last = e;
@@ -107,8 +111,11 @@ cudaError_t launch(const void* f) {
   std::lock_guard<std::recursive_mutex> lk(mu);
   const std::string name = names().count(f) ? names()[f] : "?";
   launched()[name]++;
-  if (name.find("k_fused") != std::string::npos) clock_ns += knobs()["pass_ns"];
-  if (name.find("k_update") != std::string::npos) clock_ns += knobs()["update_ns"];
+  const long long ns = name.find("k_fused") != std::string::npos    ? knobs()["pass_ns"]
+                       : name.find("k_update") != std::string::npos ? knobs()["update_ns"]
+                                                                    : 0;
+  (capturing ? captured_ns : clock_ns) += ns;
+  if (!capturing && knobs()["real_time"]) std::this_thread::sleep_for(std::chrono::nanoseconds(ns));
   if (capturing) largest = std::max(largest, ++captured);
   return cudaSuccess;
 }
@@ -278,23 +285,28 @@ cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) {
 
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) {
   ++capturing;
-  captured = 0;
+  captured = captured_ns = 0;
   return cudaSuccess;
 }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
   --capturing;
-  *g = reinterpret_cast<cudaGraph_t>(8);
+  *g = reinterpret_cast<cudaGraph_t>(captured_ns + 1);  // (a graph's handle is its time)
   return cudaSuccess;
 }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned long long) {
   if (refuse("fail_instantiate")) return ret(cudaErrorMemoryAllocation);
   std::lock_guard<std::recursive_mutex> lk(mu);
   ++instantiated;
-  *e = reinterpret_cast<cudaGraphExec_t>(8);
+  *e = reinterpret_cast<cudaGraphExec_t>(g);
   return cudaSuccess;
 }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) {
-  return refuse("fail_graph_launch") ? ret(cudaErrorMemoryAllocation) : cudaSuccess;
+cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
+  if (refuse("fail_graph_launch")) return ret(cudaErrorMemoryAllocation);
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  const long long ns = (long long)reinterpret_cast<uintptr_t>(e) - 1;
+  clock_ns += ns;
+  if (knobs()["real_time"]) std::this_thread::sleep_for(std::chrono::nanoseconds(ns));
+  return cudaSuccess;
 }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }

@@ -197,3 +197,37 @@ def test_small_shares_of_the_device():
         assert b.launch_info()["staged"] == 5
         assert np.array_equal(np.stack(a.read_fields()), np.stack(b.read_fields()))
         assert np.array_equal(a.probe_traces(), b.probe_traces())
+
+
+@pytest.mark.parametrize("every,decay", [(0, None), (10, None), (50, 30.0)])
+def test_batches_that_change_their_route(every, decay):
+    """The first spans of a set of grids run as fused passes and as shared
+    launches in turn; engines that end early leave both."""
+    scs = []
+    for k, (dims, layers) in enumerate((((23, 22, 21 + every % 7), (4,) * 6), ((17, 30, 26), None), ((21, 20, 35), (5, 0, 4, 4, 0, 5)))):
+        sc = Scenario(f"route_{k}", dims, 1e-3, excitations=[
+            oe.Excitation.gaussian_pulse(8e-12, 4e-12, 2, tuple(d // 2 for d in dims))], num_steps=2000,
+            probes=[(2, tuple(d // 2 + 2 for d in dims)), (4, (3, 3, 3))])
+        sc.cpml = oe.CpmlBoundaries(layers=layers) if layers else None
+        scs.append(sc)
+
+    def batch(sc, op, start, n):
+        b = _batch(sc, op, start, n, decay)
+        b.energy_monitoring = oe.EnergyMonitorConfig(sample_interval=every, track_peak=True)
+        return b
+    alone, packed = [_engine(sc) for sc in scs], [_engine(sc) for sc in scs]
+    pack = oe.Pack([e for _, e in packed])
+    start = 0
+    for n in (301, 500, 700):
+        on = [a.current_timestep() == start for _, a in alone]
+        got = pack.run_batch([batch(sc, op, start, n) if o else None for sc, (op, _), o in zip(scs, packed, on)])
+        for sc, (op, a), (_, b), g, o in zip(scs, alone, packed, got, on):
+            if not o:
+                continue
+            w = a.run_batch(batch(sc, op, start, n))
+            assert g.timesteps_executed == w.timesteps_executed and g.termination_reason == w.termination_reason
+            assert [(s.timestep, s.e_energy, s.h_energy) for s in g.energy_samples] == \
+                   [(s.timestep, s.e_energy, s.h_energy) for s in w.energy_samples]
+            assert np.array_equal(a.probe_traces(), b.probe_traces())
+            assert np.array_equal(np.concatenate(a.read_fields()), np.concatenate(b.read_fields()))
+        start += n

@@ -443,3 +443,35 @@ def test_column_gather_form(child, b, t, c, wide):
     N.check(L.oems_pk_col2im_causal(at[0], 5 * {c}, at[1], {b}, {t}, {c}, 5, 2, None))
     assert (launched("k_col2im_causal4") == 1) == {wide} and launched("k_col2im_causal") == 1
     """)
+
+
+@pytest.mark.parametrize("update_us,fused_wins", [(150, True), (12, False)])
+@pytest.mark.parametrize("every", [0, 10])
+def test_packs_take_the_faster_route(child, update_us, fused_wins, every):
+    """Three engines: 3 x 50 us a pass of two steps, or two shared launches a
+    step; run by one, then by the other, on the clock."""
+    child(f"""
+    knob("pass_ns", 50000), knob("update_ns", {update_us} * 1000)
+    def batches(n):
+        return [oe.EngineBatch(num_steps=n, energy_monitoring=oe.EnergyMonitorConfig(sample_interval={every}, track_peak=True))] * 3
+    def make():
+        return [engine((20, 21, 22 + k)) for k in range(3)]
+    def route(p, n):  # a length of its own is launched or captured anew
+        launched("", True)
+        p.run_batch(batches(n))
+        f, u = launched("k_fused"), launched("k_update_h_pack")
+        assert (f > 0) != (u > 0), (f, u)
+        return f > 0
+    es = make()
+    p = oe.Pack(es)
+    knob("real_time", 1)
+    for n in (300, 300, 300):
+        p.run_batch(batches(n))
+    assert launched("k_fused") > 0 and launched("k_update_h_pack") > 0  # both have run
+    assert es[2].current_timestep() == 900
+    assert route(p, 23) == {fused_wins}
+    launched("", True)
+    fs = make()
+    q = oe.Pack(fs)  # another pack of such grids: no tuning, no clock
+    assert route(q, 37) == {fused_wins} and launched("k_update") < 100
+    """)

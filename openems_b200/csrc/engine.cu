@@ -609,6 +609,8 @@ struct FusedHost {
   DevBuf<int> src_i;         // plane offsets, keys, element / direction / kind
   DevBuf<long long> src_q;   // first sample and sample count
   int src_lo = 0, src_hi = 0;
+  std::vector<int> sent_i;  // contents of src_i and src_q
+  std::vector<long long> sent_q;
   DevBuf<int> tap_i;
   int ntap = 0, tap_lo = 0, tap_hi = 0;
   DevBuf<float> taps;

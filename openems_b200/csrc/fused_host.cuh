@@ -759,7 +759,9 @@ static oems_status fused_spans(oems_engine* en, const oems_batch* b, uint64_t* c
 }
 
 // Sources of the batch sorted by (plane, row, chunk); equal cells keep the
-// list's order, which is the order they are applied in.
+// list's order, which is the order they are applied in.  Tables equal to the
+// last batch's are there already: batches of a step or two, one after the
+// other, took up to 10 us longer for sending them.
 static oems_status fused_upload_sources(oems_engine* en, const oems_batch* b, const std::vector<long long>& first,
                                         const std::vector<long long>& count) {
   FusedHost& F = en->fus;
@@ -790,11 +792,15 @@ static oems_status fused_upload_sources(oems_engine* en, const oems_batch* b, co
   if (F.src_i.n < I.size() || F.src_q.n < Q.size() || lo != F.src_lo || hi != F.src_hi) en->graph_epoch++;
   F.src_lo = lo;
   F.src_hi = hi;
+  if (F.src_i.p && F.src_q.p && I == F.sent_i && Q == F.sent_q) return OEMS_OK;
+  F.sent_i.clear();
   OEMS_CUDA(F.src_i.ensure(I.size()));
   OEMS_CUDA(F.src_q.ensure(Q.size()));
   OEMS_CUDA(cudaMemcpyAsync(F.src_i.p, I.data(), I.size() * sizeof(int), cudaMemcpyHostToDevice, en->stream));
   OEMS_CUDA(cudaMemcpyAsync(F.src_q.p, Q.data(), Q.size() * sizeof(long long), cudaMemcpyHostToDevice, en->stream));
-  OEMS_CUDA(cudaStreamSynchronize(en->stream));  // the vectors end here
+  OEMS_CUDA(cudaStreamSynchronize(en->stream));
+  F.sent_i.swap(I);
+  F.sent_q.swap(Q);
   return OEMS_OK;
 }
 

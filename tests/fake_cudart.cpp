@@ -53,7 +53,7 @@ std::map<void*, Block>& blocks() {
   static std::map<void*, Block> m;
   return m;
 }
-long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, instantiated = 0, captured = 0, largest = 0;
+long long direct = 0, pooled = 0, reserved = 0, streams = 0, pinned = 0, pins = 0, copies = 0, instantiated = 0, captured = 0, largest = 0;
 long long clock_ns = 0;  // of the launches so far
 thread_local cudaError_t last = cudaSuccess;
 thread_local int capturing = 0;
@@ -141,6 +141,7 @@ long long fake_launched(const char* part, int reset) {
 long long fake_pool_used() { return pooled; }
 long long fake_pinned() { return pinned; }  // bytes now
 long long fake_pins() { return pins; }      // calls so far
+long long fake_copies() { return copies; }  // linear ones, asked for so far
 long long fake_instantiated() { return instantiated; }
 long long fake_largest_graph() { return largest; }  // kernels in it
 
@@ -208,6 +209,7 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
   return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+  ++copies;
   return cudaMemcpy(d, s, n, k);
 }
 cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind,

@@ -475,3 +475,24 @@ def test_packs_take_the_faster_route(child, update_us, fused_wins, every):
     q = oe.Pack(fs)  # another pack of such grids: no tuning, no clock
     assert route(q, 37) == {fused_wins} and launched("k_update") < 100
     """)
+
+
+def test_source_tables_are_sent_when_they_change(child):
+    child("""
+    def run(e, n, cells):
+        dt = 1e-12
+        x = [oe.Excitation.gaussian_pulse(1e-11, 1e-11, 2, c) for c in cells]
+        before = F.fake_copies()
+        e.run_batch(oe.EngineBatch(num_steps=n, excitations=[oe.ScheduledExcitation.from_excitation(q, 0, n, dt) for q in x]))
+        return F.fake_copies() - before
+    F.fake_copies.restype = ctypes.c_longlong
+    e = engine((20, 21, 22), autotune=False)
+    a, b = [(3, 4, 5), (6, 7, 8)], [(3, 4, 5), (6, 7, 9)]
+    run(e, 2, a)
+    again = run(e, 2, a)
+    assert run(e, 2, a) == again
+    assert run(e, 2, b) == again + 2  # two tables
+    assert run(e, 2, b) == again
+    assert run(e, 3, b) == again + 2  # other sample counts
+    assert run(e, 2, a) == again + 2
+    """)

@@ -621,16 +621,19 @@ static oems_status fused_tune(oems_engine* en, bool* ok) {
       fused_release(en);
       return OEMS_OK;
     }
-    // shorter passes only finish odd spans
+    // shorter passes only finish odd spans; but batches of a step are all theirs,
+    // and below kFusedSmall the first three of the model are not the best: 64^3
+    // with CPML 21.7 us, 15.1 of 30; 100^3 18.9, 13.6; 60 x 100 x 75 11.6, 8.3 (above:
+    // the same at 128^3 to 200^3)
     const bool small = en->ncells_padded < kFusedSmall;
-    const size_t most = cached || !time_it ? 1 : steps != longest ? 3 : small ? 30 : 12;
+    const size_t most = cached || !time_it ? 1 : small ? 30 : steps != longest ? 3 : 12;
     if (c.size() > most) c.resize(most);
     FusedPlan best = c[0];
     if (c.size() > 1 || (steps == longest && time_it && !cached)) {
       float best_ms = 1e30f;
       for (FusedPlan& p : c) {
-        // (a one-step pass has a hook or a recorder before it, not another pass)
-        const bool early = longest > 1;
+        // (a one-step pass has a hook, a recorder or another batch before it, not a pass like it)
+        const bool early = steps > 1;
         OEMS_CUDA(launch_fused(en, p, 0, false, early));
         const int kReps = (int)std::max<long long>(3, std::min<long long>(8, 24000000 / en->ncells_padded));
         OEMS_CUDA(cudaEventRecord(en->ev0, en->stream));

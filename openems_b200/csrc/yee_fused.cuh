@@ -353,6 +353,16 @@ __device__ __forceinline__ int fused_find(const int* keys, int lo, int hi, int k
   return lo;
 }
 
+// Whether plane i holds entries of a table over the planes [lo, hi): only such
+// planes pay for the calls below and their copies of the cell's values.  Every
+// plane between the first and the last probe did: 128^3 with CPML, a source and
+// two probes 50.5 us a step, 38.7 now, and a batch of one step 134 us, 110 now
+// (the separate kernels 113); 256^3 with CPML 207 -> 198.  The two loads a plane
+// show on the smallest grids only (20^3 5.2 -> 5.7 us a step).
+__device__ __forceinline__ bool fused_any(const int* off, int lo, int hi, int i) {
+  return i >= lo && i < hi && __ldg(off + i + 1) > __ldg(off + i);
+}
+
 // Sources of plane i, pass step `s` (batch step): e = or += the sample, in
 // list order.
 template <typename T>
@@ -618,8 +628,8 @@ __device__ __forceinline__ void fused_item(const FusedArgs& a, const FusedBox& B
       fused_apply<kIdBytes, false, kCpml>(tab, w0, w1, d, live, e1);
 #pragma unroll
       for (int m = 0; m < 3; ++m) CIO::round(e1[m]);
-      if (i >= a.src_lo && i < a.src_hi) with_copy(e1, [&](float* e) { fused_sources<T>(a, i, key, step0, e); });
-      if (i >= a.tap_lo && i < a.tap_hi && c.own && i >= i0 && i < i1)
+      if (fused_any(a.src_off, a.src_lo, a.src_hi, i)) with_copy(e1, [&](float* e) { fused_sources<T>(a, i, key, step0, e); });
+      if (c.own && i >= i0 && i < i1 && fused_any(a.tap_off, a.tap_lo, a.tap_hi, i))
         with_copy(e1, [&](float* e) { with_copy(h1, [&](float* h) { fused_taps(a, i, key, a.local, e, h); }); });
       if constexpr (kSteps == 1) {
         if (c.own && i >= i0) {
@@ -761,8 +771,8 @@ __device__ __forceinline__ void fused_item(const FusedArgs& a, const FusedBox& B
         fused_apply<kIdBytes, false, kCpml>(tab, v0, v1, d, live, e2);
 #pragma unroll
         for (int m = 0; m < 3; ++m) CIO::round(e2[m]);
-        if (p >= a.src_lo && p < a.src_hi) with_copy(e2, [&](float* e) { fused_sources<T>(a, p, key, step0 + 1, e); });
-        if (p >= a.tap_lo && p < a.tap_hi && c.own)
+        if (fused_any(a.src_off, a.src_lo, a.src_hi, p)) with_copy(e2, [&](float* e) { fused_sources<T>(a, p, key, step0 + 1, e); });
+        if (c.own && fused_any(a.tap_off, a.tap_lo, a.tap_hi, p))
           with_copy(e2, [&](float* e) { with_copy(h2, [&](float* h) { fused_taps(a, p, key, a.local + 1, e, h); }); });
         if (c.own) {
           T* o = out + p * a.plane;

@@ -620,7 +620,8 @@ OEMS_API oems_status oems_field_energy_noalloc(const float* const fields[6], uin
 /* Per-kernel timing: while enabled, run_batch launches the update kernels one
  * by one (no graphs) with CUDA events around every H and E launch on the
  * engine's stream, and accumulates their device time.  Enabling resets the
- * totals. */
+ * totals.  Fused passes (oems_engine_launch_info) have no halves: each pass'
+ * time and count go to the H totals, and the E totals stay 0. */
 OEMS_API oems_status oems_engine_set_kernel_profiling(oems_engine* engine, int32_t enable);
 /* Launch shape chosen for the update kernels (valid after the first batch):
  * staged = 0 for the register kernels, 1 for the bulk-async staged kernels

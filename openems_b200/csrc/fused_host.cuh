@@ -700,7 +700,14 @@ static oems_status fused_or_separate(oems_engine* en, bool* yes) {
   const double cells = (double)en->nx * en->ny * en->nz, coefs = en->id_bytes ? en->id_bytes : 24;
   const double held = cells * (6 * en->elem + (en->id_bytes ? en->id_bytes : 48));
   if (held > 2 * kL2Bytes && pass < 2 * cells * (9 * en->elem + coefs) / kPeakBytes) return OEMS_OK;
-  if (!en->tuned) OEMS_TRY(autotune(en));
+  if (!en->tuned) {
+    // (without room for the copy of the state that tuning them saves, the passes it is)
+    void* save = nullptr;
+    if (!got_room(pool_alloc(&save, en->field_bytes() + (en->cpml.on ? en->cpml.psi.n * sizeof(float) : 0), en->stream)))
+      return OEMS_OK;
+    OEMS_CUDA(cudaFreeAsync(save, en->stream));
+    OEMS_TRY(autotune(en));
+  }
   *yes = !(best_of_report(en->tune_report, false, 0) < pass);
   en->tune_report.insert(en->tune_report.begin(), passes.begin(), passes.end());
   if (!*yes) {

@@ -497,3 +497,16 @@ def test_source_tables_are_sent_when_they_change(child):
     assert run(e, 3, b) == again + 2  # other sample counts
     assert run(e, 2, a) == again + 2
     """)
+
+
+def test_no_room_to_time_the_separate_kernels_keeps_the_passes(child):
+    """Tuning them saves fields and psi in one block; the passes' own buffers
+    are smaller."""
+    child("""
+    e = engine((60, 61, 64), (8,) * 6)
+    e.add_mur(oe.MurAbcConfig.all(1))
+    knob("fail_pool_from", 24 * 60 * 61 * 64 + 4096)
+    knob("pass_ns", 10 ** 9)
+    e.run_batch(batch(4))
+    assert fused(e)
+    """)
